@@ -39,6 +39,20 @@ def test_cost_matches_oracle():
     assert (wp > 0).any(), "the workload should touch obstacles"
 
 
+@pytest.mark.parametrize("Ms", [1, 63, 64, 65, 129])
+def test_cost_over_obstacle_chunks(Ms):
+    """A lane tests its obstacles 32 at a time: counts around one and two chunks of a 4-lane group's
+    share (4 x 32 = 128 obstacles) and partial ones, every sphere of the scene within reach."""
+    w, _ = setup(Bt=2, T=6)
+    w.world.spheres = W.random_sphere_world(np.random.default_rng(Ms), Ms, lo=-0.4, hi=0.4)
+    tc = TrajectoryCost(w.model, w.spheres, w.world, w.link_pairs, margin=w.margin, w_smooth=0.0, w_acc=0.0,
+                        w_jerk=0.0, w_limits=0.0, w_coll=1.0, device=DEV)
+    c = tc.cost(torch.as_tensor(w.traj, device=DEV)).cpu().numpy()
+    ref = np.array([otr.collision_cost(w.traj[b], w.model.as_dict(), w.spheres.centers, w.spheres.radii, w.link_pairs,
+                                       w.world.arrays(), w.margin) for b in range(2)])
+    np.testing.assert_allclose(c, ref, rtol=1e-4, atol=1e-5)
+
+
 def test_gradient_matches_finite_differences():
     w, tc = setup(Bt=3, T=12)
     x = torch.as_tensor(w.traj, device=DEV)
