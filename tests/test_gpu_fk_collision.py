@@ -50,7 +50,7 @@ def run_fk(g, cfg):
 
 
 @pytest.mark.parametrize("name", ["chain7", "bimanual15", "humanoid29", "odd6"])
-@pytest.mark.parametrize("B", [1, 16, 129, 4096])
+@pytest.mark.parametrize("B", [1, 16, 129, 4096, 148 * 32 + 33])
 def test_fk_cuda_matches_oracle(golden, name, B):
     g = {k: golden[f"fk_{name}_{k}"] for k in ("twists", "parent_tf", "parent_idx", "act_idx", "mimic_mul",
                                                 "mimic_off", "mimic_act_idx", "topo_inv", "lower", "upper")}
