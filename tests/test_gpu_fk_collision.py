@@ -141,6 +141,46 @@ def test_world_sphere_and_reduced(world_kind):
     assert_distances(red, rref, quantity="signed distance (collision_world_sphere_reduced)", case=world_kind)
 
 
+@pytest.mark.parametrize("S,N,Ms", [(1, 3, 1), (2, 65, 129), (13, 30, 201), (70, 90, 37)])
+def test_packed_links_over_sizes(S, N, Ms):
+    """The packed per-link kernels at odd and even sphere counts, links without spheres, obstacle
+    quads around one warp's 128, and (70 x 90 spheres) a robot that takes the unpacked kernels."""
+    rng = np.random.default_rng(S)
+    B = 5
+    c, r = sphere_robot_batch(rng, B, S, N, pad_frac=0.4)
+    r[:, :, 1] = -1e9
+    world = mixed_world(rng, Ms=Ms, Mc=1, Mb=2, Mh=1)
+    centers = np.ascontiguousarray(c.reshape(B, S * N, 3).transpose(2, 0, 1))
+    red = collision_world_sphere_reduced(tt(centers), tt(r.reshape(B, -1)), *[tt(x) for x in world], n=N).cpu().numpy()
+    ref = oc.world_sphere_reduced(c.reshape(B, S * N, 3).astype(np.float64), r.reshape(B, -1),
+                                  *[x.astype(np.float64) for x in world], N)
+    assert_distances(red, ref, quantity="signed distance (collision_world_sphere_reduced)", case=f"{S} x {N}, {Ms}")
+    pairs = np.array([(i, j) for i in range(min(N, 12)) for j in range(i)] + [(0, N), (-1, 0)], np.int32)
+    out = collision_self_sphere(tt(c), tt(r), tt(pairs[:, 0], torch.int32), tt(pairs[:, 1], torch.int32)).cpu().numpy()
+    assert (out[:, -2:] == 1e9).all()
+    ref = oc.self_sphere_full(c.astype(np.float64), r.astype(np.float64), pairs[:-2, 0], pairs[:-2, 1])
+    assert_distances(out[:, :-2], ref, quantity="signed distance (collision_self_sphere)", case=f"{S} x {N}")
+
+
+def test_packed_links_with_nan_and_infinity():
+    """A NaN or infinite centre or radius loses every minimum, as in the unpacked kernels."""
+    rng = np.random.default_rng(3)
+    B, S, N = 2, 3, 4
+    c, r = sphere_robot_batch(rng, B, S, N, pad_frac=0.0)
+    world = (W.random_sphere_world(rng, 9), np.zeros((0, 7), np.float32), np.zeros((0, 15), np.float32),
+             np.zeros((0, 6), np.float32))
+    bad_c, bad_r = c.copy(), r.copy()
+    bad_c[0, 1, 0, 0], bad_c[0, 1, 1, 2], bad_r[0, 1, 2] = np.nan, np.inf, np.nan
+    keep_r = r.copy()
+    keep_r[0, 1, :3] = -1e9
+    pi, pj = tt(np.array([0, 1, 2]), torch.int32), tt(np.array([3, 3, 1]), torch.int32)
+    soa = lambda a: tt(np.ascontiguousarray(a.reshape(B, S * N, 3).transpose(2, 0, 1)))  # noqa: E731
+    for a, b in ((collision_world_sphere_reduced(soa(bad_c), tt(bad_r.reshape(B, -1)), *[tt(x) for x in world], n=N),
+                  collision_world_sphere_reduced(soa(c), tt(keep_r.reshape(B, -1)), *[tt(x) for x in world], n=N)),
+                 (collision_self_sphere(tt(bad_c), tt(bad_r), pi, pj), collision_self_sphere(tt(c), tt(keep_r), pi, pj))):
+        np.testing.assert_array_equal(a.cpu().numpy(), b.cpu().numpy())
+
+
 def test_world_capsule_robot():
     rng = np.random.default_rng(12)
     B, N = 19, 5
