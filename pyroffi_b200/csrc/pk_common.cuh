@@ -209,15 +209,42 @@ __device__ inline void load_joint_table(JointTable& jt, const ModelArgs& m) {
       jt.axis[i][0] = jt.axis[i][1] = jt.axis[i][2] = 0.f;
     }
   }
-  if (threadIdx.x == 0) jt.n = n;
-  __syncthreads();
+  bool mine = true;  // this thread's joints follow one another
+  for (int i = threadIdx.x; i < n; i += blockDim.x) mine = mine && jt.psorted[i] == i - 1;
+  const int chain = __syncthreads_and(mine);
   if (threadIdx.x == 0) {
-    int chain = 1;
-    for (int i = 0; i < n; ++i)
-      if (jt.psorted[i] != i - 1) { chain = 0; break; }
+    jt.n = n;
     jt.chain = chain;
   }
   __syncthreads();
+}
+
+// Stable grouping of robot spheres (sphere k on joint joint[k]; out-of-range
+// joints are dropped) by sorted joint position, one sphere or joint per
+// thread: each reads all the joints, which the block's threads share through
+// L1, instead of one thread counting them in turn.
+__device__ __forceinline__ int sphere_key(const int* joint, int k, const JointTable& jt, int nj) {
+  const int j = joint[k];
+  return (j >= 0 && j < nj) ? jt.sorted_of[j] : -1;
+}
+// spheres carried by sorted joint js
+__device__ inline int spheres_on_joint(const int* joint, int n_rs, const JointTable& jt, int nj, int js) {
+  int c = 0;
+#pragma unroll 4
+  for (int k = 0; k < n_rs; ++k) c += sphere_key(joint, k, jt, nj) == js;
+  return c;
+}
+// place of sphere k among the grouped spheres (-1: dropped)
+__device__ inline int sphere_place(const int* joint, int n_rs, const JointTable& jt, int nj, int k) {
+  const int key = sphere_key(joint, k, jt, nj);
+  if (key < 0) return -1;
+  int at = 0;
+#pragma unroll 4
+  for (int q = 0; q < n_rs; ++q) {
+    const int kq = sphere_key(joint, q, jt, nj);
+    at += (kq >= 0 && (kq < key || (kq == key && q < k))) ? 1 : 0;
+  }
+  return at;
 }
 
 __device__ __forceinline__ Pose load_ptf(const JointTable& jt, int i) {

@@ -210,9 +210,12 @@ __device__ void wide_stage_class(const WideLaunch& P, const WideArgs& A, unsigne
   for (int i = tid; i < w.Ms; i += blockDim.x) ws4[i].w = ws4[i].w + P.margin;
   __syncthreads();
 
-  // Thread 0: active columns and their joint lists, FK levels, spheres
-  // grouped by joint (invalid joint indices dropped, as the reference skips
-  // them), bounding spheres, self pairs in grouped indices, grid bounds.
+  // Spheres grouped by joint (invalid joint indices dropped, as the reference
+  // skips them) and their bounding spheres by all threads; active columns and
+  // their joint lists, FK levels, self pairs in grouped indices by thread 0.
+  for (int j = tid; j < nj; j += blockDim.x)
+    sh.jstart[j + 1] = spheres_on_joint(A.sphere_joint, A.n_rs, sh.jt, nj, j);  // counts, for now
+  __syncthreads();
   if (tid == 0) {
     const JointTable& jt = sh.jt;
     const int n = jt.n;
@@ -254,54 +257,54 @@ __device__ void wide_stage_class(const WideLaunch& P, const WideArgs& A, unsigne
     sh.lvl_start[n_lvl] = run;
     for (int i = 0; i < n; ++i) sh.lvl_joint[cnt[lvl[i]]++] = i;
     sh.n_lvl = n_lvl;
-    // spheres grouped by sphere-carrying joint, in sorted joint order
-    int scnt[PK_MAX_JOINTS], slot_of[PK_MAX_JOINTS];
-    for (int j = 0; j < n; ++j) scnt[j] = 0;
-    for (int k = 0; k < A.n_rs; ++k) {
-      const int j = A.sphere_joint[k];
-      if (j >= 0 && j < nj) scnt[jt.sorted_of[j]]++;
-    }
+    // sphere-carrying joints in sorted order; jstart goes from counts (at
+    // js + 1) to offsets (at n_js <= js) in place
     int n_js = 0, total = 0;
     for (int js = 0; js < n; ++js) {
-      slot_of[js] = -1;
-      if (scnt[js] == 0) continue;
-      slot_of[js] = n_js;
+      const int c = sh.jstart[js + 1];
+      if (c == 0) continue;
       sh.js_joint[n_js] = js;
       sh.jstart[n_js] = total;
-      total += scnt[js];
-      scnt[js] = sh.jstart[n_js];
+      total += c;
       ++n_js;
     }
     sh.jstart[n_js] = total;
     sh.n_js = n_js;
     sh.n_rs = total;
-    for (int k = 0; k < A.n_rs; ++k) {
-      const int j = A.sphere_joint[k];
-      if (j < 0 || j >= nj) { rsk[k] = -1; continue; }
-      const int js = jt.sorted_of[j];
-      const int at = scnt[js]++;
-      rsk[k] = at;
-      rs4[at] = make_float4(A.spheres_local[4 * k], A.spheres_local[4 * k + 1], A.spheres_local[4 * k + 2],
-                            A.spheres_local[4 * k + 3]);
-      rsj[at] = slot_of[js];
+  }
+  __syncthreads();
+  for (int k = tid; k < A.n_rs; k += blockDim.x) {
+    const int at = sphere_place(A.sphere_joint, A.n_rs, sh.jt, nj, k);
+    rsk[k] = at;
+    if (at < 0) continue;
+    rs4[at] = make_float4(A.spheres_local[4 * k], A.spheres_local[4 * k + 1], A.spheres_local[4 * k + 2],
+                          A.spheres_local[4 * k + 3]);
+    const int key = sphere_key(A.sphere_joint, k, sh.jt, nj);
+    int slot = 0;
+    while (sh.js_joint[slot] != key) ++slot;  // key carries a sphere, so it is listed
+    rsj[at] = slot;
+  }
+  __syncthreads();
+  const int n_js = sh.n_js;
+  for (int q = tid; q < n_js; q += blockDim.x) {
+    float lo3[3] = {3e38f, 3e38f, 3e38f}, hi3[3] = {-3e38f, -3e38f, -3e38f};
+    for (int k = sh.jstart[q]; k < sh.jstart[q + 1]; ++k) {
+      const float v[3] = {rs4[k].x, rs4[k].y, rs4[k].z};
+      for (int d = 0; d < 3; ++d) { lo3[d] = fminf(lo3[d], v[d]); hi3[d] = fmaxf(hi3[d], v[d]); }
     }
+    const float cx = 0.5f * (lo3[0] + hi3[0]), cy = 0.5f * (lo3[1] + hi3[1]), cz = 0.5f * (lo3[2] + hi3[2]);
+    float R = -3e38f;
+    for (int k = sh.jstart[q]; k < sh.jstart[q + 1]; ++k) {
+      const float dx = rs4[k].x - cx, dy = rs4[k].y - cy, dz = rs4[k].z - cz;
+      R = fmaxf(R, sqrtf(dx * dx + dy * dy + dz * dz) + rs4[k].w);
+    }
+    R = R + 1e-4f + 1e-5f * fabsf(R);  // slack keeps the cull conservative under FP32 rounding
+    sh.jb[q] = make_float4(cx, cy, cz, R);
+  }
+  __syncthreads();
+  if (tid == 0) {
     float rmax = 0.f;
-    for (int q = 0; q < n_js; ++q) {
-      float lo3[3] = {3e38f, 3e38f, 3e38f}, hi3[3] = {-3e38f, -3e38f, -3e38f};
-      for (int k = sh.jstart[q]; k < sh.jstart[q + 1]; ++k) {
-        const float v[3] = {rs4[k].x, rs4[k].y, rs4[k].z};
-        for (int d = 0; d < 3; ++d) { lo3[d] = fminf(lo3[d], v[d]); hi3[d] = fmaxf(hi3[d], v[d]); }
-      }
-      const float cx = 0.5f * (lo3[0] + hi3[0]), cy = 0.5f * (lo3[1] + hi3[1]), cz = 0.5f * (lo3[2] + hi3[2]);
-      float R = -3e38f;
-      for (int k = sh.jstart[q]; k < sh.jstart[q + 1]; ++k) {
-        const float dx = rs4[k].x - cx, dy = rs4[k].y - cy, dz = rs4[k].z - cz;
-        R = fmaxf(R, sqrtf(dx * dx + dy * dy + dz * dz) + rs4[k].w);
-      }
-      R = R + 1e-4f + 1e-5f * fabsf(R);  // slack keeps the cull conservative under FP32 rounding
-      sh.jb[q] = make_float4(cx, cy, cz, R);
-      rmax = fmaxf(rmax, R);
-    }
+    for (int q = 0; q < n_js; ++q) rmax = fmaxf(rmax, sh.jb[q].w);
     sh.rmax = rmax;
     // self pairs in grouped sphere positions (pairs with an invalid sphere are dropped)
     int n_pairs = 0;
@@ -317,22 +320,21 @@ __device__ void wide_stage_class(const WideLaunch& P, const WideArgs& A, unsigne
     // obstacle-grid bounds (world radii already carry the margin)
     sh.grid_on = 0;
     sh.grid_n = L.grid_n;
-    if (L.max_entries > 0 && n_js > 0 && P.coll) {
-      obstacle_grid_bounds(ws4, w.Ms, rmax, sh.grid_n, sh.glo, sh.ginv);
-      sh.grid_on = 1;
-    }
+    if (L.max_entries > 0 && n_js > 0 && P.coll) sh.grid_on = 1;
   }
   __syncthreads();
 
   if (sh.grid_on) {
+    if (tid < 32) obstacle_grid_bounds(ws4, w.Ms, sh.rmax, L.grid_n, sh.glo, sh.ginv);
+    __syncthreads();
     obstacle_grid_build(ws4, w.Ms, sh.rmax, sh.grid_n, sh.glo, sh.ginv, obox, cell_start, cell_obs, L.max_entries,
                         sh.grid_on);
     // a fine grid whose lists overflow the capacity falls back to the default resolution
     if (!sh.grid_on && sh.grid_n > kObsGridDefault) {
       __syncthreads();
-      if (threadIdx.x == 0) {
+      if (tid < 32) obstacle_grid_bounds(ws4, w.Ms, sh.rmax, kObsGridDefault, sh.glo, sh.ginv);
+      if (tid == 0) {
         sh.grid_n = kObsGridDefault;
-        obstacle_grid_bounds(ws4, w.Ms, sh.rmax, sh.grid_n, sh.glo, sh.ginv);
         sh.grid_on = 1;
       }
       __syncthreads();

@@ -44,27 +44,41 @@ __host__ __device__ __forceinline__ int obstacle_grid_capacity(int G, int Ms) {
   return c < 1024 ? 1024 : (c > 16384 ? 16384 : c);
 }
 
-// Origin and inverse cell size of the grid (one thread).
+// Origin and inverse cell size of the grid, by the 32 lanes of one warp (lane
+// 0 writes them).
 __device__ inline void obstacle_grid_bounds(const float4* ws, int Ms, float reach, int G, float3& lo, float3& inv) {
   float l[3] = {3e38f, 3e38f, 3e38f}, h[3] = {-3e38f, -3e38f, -3e38f};
-  for (int o = 0; o < Ms; ++o) {
+  const int lane = threadIdx.x & 31;
+  for (int o = lane; o < Ms; o += 32) {
     const float4 O = ws[o];
     const float rho = O.w + reach + 1e-3f;
     l[0] = fminf(l[0], O.x - rho); h[0] = fmaxf(h[0], O.x + rho);
     l[1] = fminf(l[1], O.y - rho); h[1] = fmaxf(h[1], O.y + rho);
     l[2] = fminf(l[2], O.z - rho); h[2] = fmaxf(h[2], O.z + rho);
   }
-  lo = make_float3(l[0], l[1], l[2]);
-  inv = make_float3(G / fmaxf(h[0] - l[0], 1e-6f), G / fmaxf(h[1] - l[1], 1e-6f), G / fmaxf(h[2] - l[2], 1e-6f));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      l[d] = fminf(l[d], __shfl_xor_sync(0xffffffffu, l[d], o));
+      h[d] = fmaxf(h[d], __shfl_xor_sync(0xffffffffu, h[d], o));
+    }
+  if (lane == 0) {
+    lo = make_float3(l[0], l[1], l[2]);
+    inv = make_float3(G / fmaxf(h[0] - l[0], 1e-6f), G / fmaxf(h[1] - l[1], 1e-6f), G / fmaxf(h[2] - l[2], 1e-6f));
+  }
 }
 
 // Cell lists: cell_start[G^3 + 1] offsets into cell_obs; obox[Ms]
 // is scratch.  Called by every thread of the block with block-uniform
-// arguments; `on` (shared) is cleared when the lists would exceed
+// arguments (blockDim a multiple of 32); `on` (shared) is cleared when the lists would exceed
 // max_entries, and the caller then scans every obstacle instead.  Each
 // obstacle adds itself to the cells of its box (shared-memory atomics), and
 // every cell's list is then sorted, so the lists hold increasing obstacle
-// indices whatever the order of the atomics.
+// indices whatever the order of the atomics.  The offsets are a scan over the
+// block, each thread taking a run of cells: by one thread alone the 2,744
+// cells of the finest default took about 0.1 ms of every block's staging
+// (with the grouping of spheres and pairs, 0.08 of 1.55 ms on the IK benchmark's 6 iterations).
 __device__ inline void obstacle_grid_build(const float4* ws, int Ms, float reach, int G, float3 lo, float3 inv,
                                            int* obox, int* cell_start, unsigned short* cell_obs, int max_entries,
                                            int& on) {
@@ -93,13 +107,27 @@ __device__ inline void obstacle_grid_build(const float4* ws, int Ms, float reach
   };
   for (int o = tid; o < Ms; o += nth) cells_of(o, [&](int c) { atomicAdd(&cell_start[c], 1); });
   __syncthreads();
-  if (tid == 0) {
-    int run = 0;
-    for (int c = 0; c < NC; ++c) {
-      const int n = cell_start[c];
-      cell_start[c] = run;
-      run += n;
-    }
+  int* const s_warp = reinterpret_cast<int*>(cell_obs);  // warp sums; the lists are filled later
+  const int per = (NC + nth - 1) / nth, c0 = min(tid * per, NC), c1 = min(c0 + per, NC);
+  const int lane = tid & 31, wid = tid >> 5;
+  int sum = 0;
+  for (int c = c0; c < c1; ++c) sum += cell_start[c];
+  int inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  if (lane == 31) s_warp[wid] = inc;
+  __syncthreads();
+  int run = inc - sum;
+  for (int w = 0; w < wid; ++w) run += s_warp[w];
+  for (int c = c0; c < c1; ++c) {
+    const int n = cell_start[c];
+    cell_start[c] = run;
+    run += n;
+  }
+  if (tid == nth - 1) {
     cell_start[NC] = run;
     if (run > max_entries) on = 0;
   }
@@ -109,10 +137,10 @@ __device__ inline void obstacle_grid_build(const float4* ws, int Ms, float reach
     for (int o = tid; o < Ms; o += nth)
       cells_of(o, [&](int c) { cell_obs[atomicAdd(&cell_start[c], 1)] = (unsigned short)o; });
     __syncthreads();
-    if (tid == 0) {
-      for (int c = NC - 1; c > 0; --c) cell_start[c] = cell_start[c - 1];
-      cell_start[0] = 0;
-    }
+    const int before = c0 > 0 ? cell_start[c0 - 1] : 0;
+    __syncthreads();
+    for (int c = c1 - 1; c > c0; --c) cell_start[c] = cell_start[c - 1];
+    if (c0 < c1) cell_start[c0] = before;
     __syncthreads();
     for (int c = tid; c < NC; c += nth) {
       const int e0 = cell_start[c], e1 = cell_start[c + 1];

@@ -127,29 +127,23 @@ __device__ inline void seed_ik_stage(const SeedIkArgs& a, SeedIkShared& sh, Robo
     sh.fixed[c] = live ? (a.fixed_mask ? a.fixed_mask[c] != 0 : 0) : 1;
   }
   __syncthreads();  // sorted_of is complete
+  // robot spheres grouped by (sorted) joint, in sphere order within a group;
+  // spheres on an out-of-range joint are dropped
+  for (int j = tid; j < nj; j += nth) R.start[j + 1] = spheres_on_joint(a.rs_joint, a.n_rs, sh.jt, nj, j);
+  for (int i = tid; i < a.n_rs; i += nth) {
+    const int at = sphere_place(a.rs_joint, a.n_rs, sh.jt, nj, i);
+    const float* q = a.rs_local + 4 * i;
+    if (at >= 0) R.sph[at] = make_float4(q[0], q[1], q[2], q[3]);
+  }
+  __syncthreads();
   if (tid == 0) {
-    // robot spheres grouped by (sorted) joint, in sphere order within a group;
-    // spheres on an out-of-range joint are dropped
-    for (int j = 0; j <= nj; ++j) R.start[j] = 0;
-    for (int i = 0; i < a.n_rs; ++i) {
-      const int j = a.rs_joint[i];
-      if (j >= 0 && j < nj) ++R.start[sh.jt.sorted_of[j] + 1];
-    }
     int ng = 0, off = 0;
     for (int j = 0; j < nj; ++j) {
       const int c = R.start[j + 1];
       if (c) { R.joint[ng] = j; R.gstart[ng] = off; ++ng; off += c; }
-      R.start[j + 1] = off;  // fill cursor base: start[j] .. start[j + 1]
     }
     R.gstart[ng] = off;
     sh.n_groups = ng;
-    // start[j] now holds where joint j's spheres begin: the fill cursor
-    for (int i = 0; i < a.n_rs; ++i) {
-      const int j = a.rs_joint[i];
-      if (j < 0 || j >= nj) continue;
-      const float* q = a.rs_local + 4 * i;
-      R.sph[R.start[sh.jt.sorted_of[j]]++] = make_float4(q[0], q[1], q[2], q[3]);
-    }
   }
   __syncthreads();
   R.ng = sh.n_groups;
@@ -195,9 +189,9 @@ __device__ inline void seed_ik_stage(const SeedIkArgs& a, SeedIkShared& sh, Robo
     float reach = 0.f;
     for (int k = 0; k < R.ng; ++k) reach = fmaxf(reach, R.bound[k].w);
     reach += a.collision_margin;
+    if (tid < 32) obstacle_grid_bounds(ob.sph, ob.Ms, reach, a.grid_n, sh.glo, sh.ginv);
     if (tid == 0) {
       sh.grid_n = a.grid_n;
-      obstacle_grid_bounds(ob.sph, ob.Ms, reach, sh.grid_n, sh.glo, sh.ginv);
       sh.grid_on = 1;
     }
     __syncthreads();
@@ -206,9 +200,9 @@ __device__ inline void seed_ik_stage(const SeedIkArgs& a, SeedIkShared& sh, Robo
     // a fine grid whose lists overflow the capacity falls back to the default resolution
     if (!sh.grid_on && sh.grid_n > kObsGridDefault) {
       __syncthreads();
+      if (tid < 32) obstacle_grid_bounds(ob.sph, ob.Ms, reach, kObsGridDefault, sh.glo, sh.ginv);
       if (tid == 0) {
         sh.grid_n = kObsGridDefault;
-        obstacle_grid_bounds(ob.sph, ob.Ms, reach, sh.grid_n, sh.glo, sh.ginv);
         sh.grid_on = 1;
       }
       __syncthreads();
