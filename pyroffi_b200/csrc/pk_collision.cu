@@ -78,18 +78,6 @@ __device__ __forceinline__ void pack_link_pairs(float4* dst, int* counts, int nc
   }
 }
 
-// sqrt(x) from the approximate reciprocal square root y of x (or of x + 1e-30)
-// and one Newton step: within an ulp, where x y alone is a few ulp off.
-__device__ __forceinline__ float root_newton(float x, float y) {
-  const float s = x * y;
-  return fmaf(fmaf(-s, s, x), 0.5f * y, s);
-}
-__device__ __forceinline__ float2 root_newton2(float2 x, float2 y) {
-  const float2 s = __fmul2_rn(x, y);
-  const float2 e = __ffma2_rn(make_float2(-s.x, -s.y), s, x);
-  return __ffma2_rn(e, __fmul2_rn(y, make_float2(0.5f, 0.5f)), s);
-}
-
 __device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
 // Signed distances of the sphere pair (A, B) to the sphere at -(nx, ny, nz),

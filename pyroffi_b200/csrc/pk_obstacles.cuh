@@ -22,6 +22,18 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 // (giving 0) and is below FP32 resolution for any x above 1e-23.
 __device__ __forceinline__ float sqrt_fast(float x) { return x * rsqrt_approx(x + 1e-30f); }
 
+// sqrt(x) from the approximate reciprocal square root y of x (or of x + 1e-30)
+// and one Newton step: within an ulp, where x y alone is a few ulp off.
+__device__ __forceinline__ float root_newton(float x, float y) {
+  const float s = x * y;
+  return fmaf(fmaf(-s, s, x), 0.5f * y, s);
+}
+__device__ __forceinline__ float2 root_newton2(float2 x, float2 y) {
+  const float2 s = __fmul2_rn(x, y);
+  const float2 e = __ffma2_rn(make_float2(-s.x, -s.y), s, x);
+  return __ffma2_rn(e, __fmul2_rn(y, make_float2(0.5f, 0.5f)), s);
+}
+
 struct WorldArgs {
   const float* spheres;
   const float* capsules;
@@ -208,13 +220,16 @@ struct LinkSpheres {
     const float2 len = __fmul2_rn(d2, make_float2(rsqrt_approx(e.x), rsqrt_approx(e.y)));
     return __ffma2_rn(__fadd2_rn(r[q], rp), make_float2(-1.f, -1.f), len);
   }
-  // d_sphere_sphere against world sphere o (IEEE sqrt)
+  // d_sphere_sphere against world sphere o (the Newton-corrected root, an ulp
+  // from the IEEE one at a third of its instructions: trajectory cost and
+  // gradient launches of 512 x 64 x 7 336 -> 293 us)
   __device__ __forceinline__ float2 sphere_dist2(int q, float4 o) const {
     const float2 d2 = sq_dist2(q, make_float2(-o.x, -o.x), make_float2(-o.y, -o.y), make_float2(-o.z, -o.z));
-    const float2 len = make_float2(sqrtf(d2.x), sqrtf(d2.y));
+    const float2 e = __fadd2_rn(d2, make_float2(1e-30f, 1e-30f));
+    const float2 len = root_newton2(d2, make_float2(rsqrt_approx(e.x), rsqrt_approx(e.y)));
     return __ffma2_rn(__fadd2_rn(r[q], make_float2(o.w, o.w)), make_float2(-1.f, -1.f), len);
   }
-  // d_sphere_box against box b (centre, axis columns, half-lengths; IEEE sqrt)
+  // d_sphere_box against box b (centre, axis columns, half-lengths; root as above)
   __device__ __forceinline__ float2 box_dist2(int q, const float* b) const {
     const float2 dx = __fadd2_rn(x[q], make_float2(-b[0], -b[0]));
     const float2 dy = __fadd2_rn(y[q], make_float2(-b[1], -b[1]));
@@ -233,7 +248,8 @@ struct LinkSpheres {
     float2 s2 = __fmul2_rn(m1, m1);
     s2 = __ffma2_rn(m2, m2, s2);
     s2 = __ffma2_rn(m3, m3, s2);
-    const float2 out = make_float2(sqrtf(s2.x), sqrtf(s2.y));
+    const float2 e = __fadd2_rn(s2, make_float2(1e-30f, 1e-30f));
+    const float2 out = root_newton2(s2, make_float2(rsqrt_approx(e.x), rsqrt_approx(e.y)));
     const float2 in = make_float2(fminf(fmaxf(fmaxf(qv[0].x, qv[1].x), qv[2].x), 0.f),
                                   fminf(fmaxf(fmaxf(qv[0].y, qv[1].y), qv[2].y), 0.f));
     return __ffma2_rn(r[q], make_float2(-1.f, -1.f), __fadd2_rn(out, in));
