@@ -101,6 +101,28 @@ def test_inner_solve_matches_oracle():
             np.testing.assert_array_equal(got[b, -1], q[0, -1])
 
 
+@pytest.mark.parametrize("T,n,m", [(2, 7, 6), (4, 7, 6), (5, 6, 6), (6, 8, 1), (32, 7, 6), (33, 7, 6), (65, 5, 3),
+                                   (128, 8, 6), (129, 7, 6), (16, 9, 6), (16, 7, 7)])
+def test_inner_solve_by_waypoint_equals_by_block(T, n, m):
+    """The thread-per-waypoint solve (up to 128 waypoints, 8 joints, a history of 6; the last three
+    are past its limits) against the block solve, which inner_threads asks for.  Eight iterations of
+    two FP32 sums in different orders: 1e-3 of the step."""
+    from pyroffi_b200.robot import random_spheres, serial_chain
+    rng = np.random.default_rng(T + n)
+    model = serial_chain(n, rng)
+    sph = random_spheres(model, rng, per_link=2)
+    B = 3
+    x = torch.as_tensor(rng.uniform(-1, 1, size=(B, T, n)), dtype=torch.float32, device=DEV)
+    d = torch.as_tensor(rng.uniform(-0.05, 0.1, size=(B, T, 5)), dtype=torch.float32, device=DEV)
+    J = torch.as_tensor(rng.normal(size=(B, T, 5, n)), dtype=torch.float32, device=DEV)
+    out = [ScoOptimizer(model, sph, W.empty_world(), np.zeros((0, 2)), ScoConfig(n_inner_iters=8, m_lbfgs=m),
+                        inner_threads=th, device=DEV).inner(x, d, J, 3.0, x[0, 0], x[0, -1]) for th in (0, 64)]
+    step = (out[1] - x)[:, 1:-1].norm() + 1e-6
+    assert torch.isfinite(out[0]).all()
+    assert (out[0] - out[1]).norm() <= 1e-3 * step
+    assert torch.equal(out[0][:, 0], x[:1, 0].expand(B, n)) and torch.equal(out[0][:, -1], x[:1, -1].expand(B, n))
+
+
 def test_final_cost_matches_oracle():
     w = scene()
     cfg = ScoConfig()
