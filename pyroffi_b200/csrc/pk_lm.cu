@@ -1378,6 +1378,7 @@ struct SeedGroupBatch {
   const int4* items;
   int n_items;
   int* queue;
+  int shift;  // the item counter is the 16 bits of *queue from here on, or all of it (32)
 };
 
 // MINB as for lm_kernel.  MAXA / MAXEE select the body: <8, 1> serves the
@@ -1389,8 +1390,11 @@ __global__ void __launch_bounds__(128, MINB) lm_batch_kernel(const __grid_consta
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int s_item;
   __shared__ LmArgs s_args;
+  batch_trigger();
   for (;;) {
-    if (threadIdx.x == 0) s_item = atomicAdd(B.queue, 1);
+    if (threadIdx.x == 0)
+      s_item = B.shift >= 32 ? atomicAdd(B.queue, 1)
+                             : (int)((atomicAdd(reinterpret_cast<unsigned*>(B.queue), 1u << B.shift) >> B.shift) & 0xffffu);
     __syncthreads();
     const int it = s_item;
     __syncthreads();
@@ -1410,6 +1414,7 @@ __global__ void __launch_bounds__(128, MINB) lm_batch_kernel(const __grid_consta
     lm_seed_groups<MAXA, MAXEE, TPS>(a, smem_raw, L, item.y, item.w, (size_t)item.y * a.Sd + item.z);
     __syncthreads();
   }
+  batch_join();
 }
 
 // ---------------------------------------------------------------------------
@@ -2124,8 +2129,12 @@ extern "C" int pk_ik_verify_select(void* stream, const float* cfgs, const float*
 
 namespace pk {
 
+// How the item counter queue[0] has been used by this call's launches so far.
+enum QueueUse { kQueueClear, kQueueHalves, kQueueWhole };
+
 template <int MAXA, int MAXEE, int TPS>
-static int launch_batch_t(const SeedGroupBatch& B, size_t smem, int threads, int blocks, cudaStream_t st) {
+static int launch_batch_t(SeedGroupBatch B, size_t smem, int threads, int blocks, cudaStream_t st, int shift,
+                          QueueUse& queue_use, bool follows) {
   // the 4-block register budget only where shared memory admits 3 or more blocks per SM (8-wide body)
   auto kern = lm_batch_kernel<MAXA, MAXEE, TPS, 2>;
   if constexpr (MAXA <= 8)
@@ -2139,14 +2148,28 @@ static int launch_batch_t(const SeedGroupBatch& B, size_t smem, int threads, int
       return s;
     blocks = std::max(1, sms * std::max(per_sm, 1));
   }
-  kern<<<blocks, threads, smem, st>>>(B);
+  // The two seed-group kernels share the counter queue[0]: 16 bits each, so
+  // that they can run side by side, where those hold every block's last,
+  // failing take too; else the whole word, cleared on the stream in between,
+  // which also keeps the second kernel from starting early.
+  const bool whole = queue_use == kQueueWhole || (long long)B.n_items + blocks >= 65536;
+  B.shift = whole ? 32 : shift;
+  if (whole && queue_use != kQueueClear) {
+    if (int s = cuda_status(cudaMemsetAsync(B.queue, 0, sizeof(int32_t), st), "queue reset")) return s;
+    follows = false;
+  }
+  queue_use = whole ? kQueueWhole : kQueueHalves;
+  if (int s = cuda_status(batch_launch(kern, dim3((unsigned)blocks), threads, smem, st, follows, B),
+                          "lm_batch_kernel launch"))
+    return s;
   return cuda_status(cudaGetLastError(), "lm_batch_kernel launch");
 }
 
 // One persistent launch over the items of the classes of `body`
 // (kBodySeedGroup: 8-wide, lanes and seeds per block from the options;
 // kBodySeedGroup16: 16-wide, one lane per seed, kSeedsPerBlock16 seeds per block).
-static int launch_seed_group_body(const BatchCall& b, int body, cudaStream_t st, bool& queue_used, int& count) {
+static int launch_seed_group_body(const BatchCall& b, int body, cudaStream_t st, QueueUse& queue_use, int& count,
+                                  bool follows) {
   int tps = b.opt.threads_per_seed, spb = b.opt.seeds_per_block;
   if (body == kBodySeedGroup16) {
     tps = 1;
@@ -2223,35 +2246,29 @@ static int launch_seed_group_body(const BatchCall& b, int body, cudaStream_t st,
   B.n_items = b.n_items;
   B.queue = b.queue;
   const int threads = spb * tps;
-  // the item counter queue[0] serves both seed-group launches: the second
-  // one starts from a counter cleared on the stream after the first
-  if (queue_used) {
-    if (int s = cuda_status(cudaMemsetAsync(b.queue, 0, sizeof(int32_t), st), "queue reset")) return s;
-  }
   int s;
   if (body == kBodySeedGroup16) {
-    s = launch_batch_t<16, 2, 1>(B, smem, threads, b.blocks, st);
+    s = launch_batch_t<16, 2, 1>(B, smem, threads, b.blocks, st, 0, queue_use, follows);
   } else {
     switch (tps) {
-      case 1: s = launch_batch_t<8, 1, 1>(B, smem, threads, b.blocks, st); break;
-      case 2: s = launch_batch_t<8, 1, 2>(B, smem, threads, b.blocks, st); break;
-      case 4: s = launch_batch_t<8, 1, 4>(B, smem, threads, b.blocks, st); break;
-      default: s = launch_batch_t<8, 1, 8>(B, smem, threads, b.blocks, st); break;
+      case 1: s = launch_batch_t<8, 1, 1>(B, smem, threads, b.blocks, st, 16, queue_use, follows); break;
+      case 2: s = launch_batch_t<8, 1, 2>(B, smem, threads, b.blocks, st, 16, queue_use, follows); break;
+      case 4: s = launch_batch_t<8, 1, 4>(B, smem, threads, b.blocks, st, 16, queue_use, follows); break;
+      default: s = launch_batch_t<8, 1, 8>(B, smem, threads, b.blocks, st, 16, queue_use, follows); break;
     }
   }
-  if (s == PK_OK) {
-    queue_used = true;
-    ++count;
-  }
+  if (s == PK_OK) ++count;
   return s;
 }
 
 int launch_seed_group_batch(const BatchCall& b, cudaStream_t st, int* launched) {
-  bool queue_used = false;
-  int n = 0;
-  if (int s = launch_seed_group_body(b, kBodySeedGroup, st, queue_used, n)) return s;
-  if (int s = launch_seed_group_body(b, kBodySeedGroup16, st, queue_used, n)) return s;
-  if (launched) *launched += n;
+  // the longer items first: what is left of an SM at the end of a body is
+  // filled by the next one
+  QueueUse queue_use = kQueueClear;
+  int n = launched ? *launched : 0;
+  if (int s = launch_seed_group_body(b, kBodySeedGroup16, st, queue_use, n, n > 0)) return s;
+  if (int s = launch_seed_group_body(b, kBodySeedGroup, st, queue_use, n, n > 0)) return s;
+  if (launched) *launched = n;
   return PK_OK;
 }
 

@@ -865,6 +865,7 @@ __global__ void __launch_bounds__(256, 2) lm_warp_kernel(const __grid_constant__
   const int group = threadIdx.x / G, gl = threadIdx.x % G, ngroups = blockDim.x / G;
   const unsigned gm = (G == 32) ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
   const WideWarp W = w_group_area(P.L, smem, group);
+  if (P.queue) batch_trigger();
   int staged_cls = -1, staged_pb = -1;
   for (int round = 0;; ++round) {
     int4 item;

@@ -131,6 +131,22 @@ def test_batch_equals_per_class_launches(mixed):
         assert np.all(np.isinf(b.out_err[c].cpu().numpy()[~m]))
 
 
+def test_batch_with_more_blocks_than_half_counters_hold(mixed):
+    """Items plus blocks past 65,535 make the two seed-group kernels take the whole item counter in
+    turn instead of 16 bits each at the same time."""
+    w = mixed
+    outs = []
+    for blocks in (0, 65536):
+        b = MixedIkBatch(w.classes, w.world, device=DEV, blocks=blocks, **opts(w, max_iter=2))
+        b.prepare(w.problem_class, w.n_seeds)
+        b.load(w.target_T, w.seeds)
+        b.run_lm()
+        outs.append((b.out_cfg, b.out_err))
+    for x, y in zip(*outs):
+        for p, q in zip(x, y):
+            assert torch.equal(p, q)
+
+
 def test_batch_graph_replay_and_reload(mixed):
     w = mixed
     b = make_batch(w)
