@@ -212,22 +212,15 @@ constexpr float kScoSkip = 20.f;
 // the collision sum wanted, its distance at or above the margin).
 template <int KIND, int MAXS, int TG>
 __device__ __forceinline__ SoftAcc world_group(const ScoLinArgs& a, const ObsView& ob, int base, int count, int gl,
-                                               unsigned gm, const LinkSpheres<MAXS>& L, float3 B, float R,
-                                               bool want_soft, bool want_j, float inv_tau, float gref,
-                                               float& csum) {
+                                               unsigned gm, const LinkSpheres<MAXS>& L, const float4* link_sph,
+                                               const Pose& Tl, float3 B, float R, bool want_soft, bool want_j,
+                                               float inv_tau, float gref, float& csum) {
   SoftAcc acc;
   acc.init();
-  for (int k = gl; k < count; k += TG) {
-    ScoObs<KIND> o;
-    o.load(ob, k);
-    const float lb = o.dist(B.x, B.y, B.z, R);  // <= every sphere distance of the link
-    if (want_soft) {
-      if (-lb * inv_tau < fmaxf(acc.ref, gref) - kScoSkip && (!a.coll || lb >= a.margin)) continue;
-    } else if (lb >= a.margin) {
-      continue;  // adds exactly 0 to the collision sum
-    }
-    float dmin = FLT_MAX;
-    int arg = 0;
+  // the link's minimum over its spheres for obstacle o, and the sphere that attains it
+  auto link_min = [&](const ScoObs<KIND>& o, float& dmin, int& arg) {
+    dmin = FLT_MAX;
+    arg = 0;
     if constexpr (KIND == 1) {
       const float2 nx = make_float2(-o.x, -o.x), ny = make_float2(-o.y, -o.y), nz = make_float2(-o.z, -o.z);
       const float2 ro = make_float2(o.r, o.r);
@@ -244,21 +237,54 @@ __device__ __forceinline__ SoftAcc world_group(const ScoLinArgs& a, const ObsVie
         if (d < dmin) { dmin = d; arg = s; }
       }
     }
+  };
+  if (!want_soft) {
+    // the collision sum alone: a pair at least the margin apart adds exactly 0
+    auto add = [&](int m, auto) {
+      ScoObs<KIND> o;
+      o.load(ob, m - base);
+      float dmin;
+      int arg;
+      link_min(o, dmin, arg);
+      csum -= colldist(dmin, a.margin);
+    };
+    near_of_kind<KIND - 1>(ob, base, count, B, R, a.margin, gl, TG, add);
+    return acc;
+  }
+  for (int k = gl; k < count; k += TG) {
+    ScoObs<KIND> o;
+    o.load(ob, k);
+    const float lb = o.dist(B.x, B.y, B.z, R);  // <= every sphere distance of the link
+    if (-lb * inv_tau < fmaxf(acc.ref, gref) - kScoSkip && (!a.coll || lb >= a.margin)) continue;
+    float dmin;
+    int arg;
+    link_min(o, dmin, arg);
     if (a.coll) csum -= colldist(dmin, a.margin);
-    if (!want_soft) continue;
     const float e = -dmin * inv_tau;
     if (e < fmaxf(acc.ref, gref) - kScoSkip) continue;
     float3 cc = make_float3(0.f, 0.f, 0.f), gg = cc;
     if (want_j) {
-      float rr = 0.f;
-#pragma unroll
-      for (int s = 0; s < MAXS; ++s)
-        if (s == arg) { cc = make_float3(L.X(s), L.Y(s), L.Z(s)); rr = L.R(s); }
-      obstacle_dist_grad<KIND - 1>(ob, base + k, cc, rr, gg);
+      // the attaining sphere, placed again from the link frame (a register
+      // array cannot be indexed by `arg`, and picking it out of MAXS costs
+      // more); with the root below and the ranking pass's survivor masks, one
+      // SCO step of 512 x 64 x 7 among 305 obstacles 1661 -> 1589 us
+      const float4 ls = link_sph[arg];
+      cc = pose_apply(Tl, make_float3(ls.x, ls.y, ls.z));
+      if constexpr (KIND == 1) {
+        // (c - o) / |c - o| by the approximate reciprocal root and one Newton
+        // step (about an ulp); 0 where the centres coincide
+        gg = make_float3(cc.x - o.x, cc.y - o.y, cc.z - o.z);
+        const float d2 = gg.x * gg.x + gg.y * gg.y + gg.z * gg.z;
+        float y = rsqrt_approx(d2 + 1e-30f);
+        y = y * fmaf(-0.5f * d2, y * y, 1.5f);
+        gg.x *= y; gg.y *= y; gg.z *= y;
+      } else {
+        obstacle_dist_grad<KIND - 1>(ob, base + k, cc, ls.w, gg);
+      }
     }
     acc.add(e, true, want_j, gg, cc);
   }
-  if (want_soft) acc.merge<TG>(gm);
+  acc.merge<TG>(gm);
   return acc;
 }
 
@@ -374,16 +400,16 @@ __global__ void __launch_bounds__(128, MAXS <= 8 ? 4 : (MAXS <= 16 ? 3 : 2)) sco
       // world groups: (link, obstacle) pairs, lane gl takes obstacles gl, gl + TG, ...
       SoftAcc mine, t;
       mine.init();
-      t = world_group<1, MAXS, TG>(a, ob, 0, Ms, gl, gm, ls, Bw, bl.w, want_soft, want_j, inv_tau,
-                                   gref[1], csum);
+      t = world_group<1, MAXS, TG>(a, ob, 0, Ms, gl, gm, ls, lsph + l * S, Tl, Bw, bl.w, want_soft,
+                                   want_j, inv_tau, gref[1], csum);
       if (gl == 1) mine = t;
-      t = world_group<2, MAXS, TG>(a, ob, Ms, Mc, gl, gm, ls, Bw, bl.w, want_soft, want_j, inv_tau,
-                                   gref[2], csum);
+      t = world_group<2, MAXS, TG>(a, ob, Ms, Mc, gl, gm, ls, lsph + l * S, Tl, Bw, bl.w, want_soft,
+                                   want_j, inv_tau, gref[2], csum);
       if (gl == 2) mine = t;
-      t = world_group<3, MAXS, TG>(a, ob, Ms + Mc, Mb, gl, gm, ls, Bw, bl.w, want_soft, want_j,
-                                   inv_tau, gref[3], csum);
+      t = world_group<3, MAXS, TG>(a, ob, Ms + Mc, Mb, gl, gm, ls, lsph + l * S, Tl, Bw, bl.w, want_soft,
+                                   want_j, inv_tau, gref[3], csum);
       if (gl == 3) mine = t;
-      t = world_group<4, MAXS, TG>(a, ob, Ms + Mc + Mb, a.w.Mh, gl, gm, ls, Bw, bl.w, want_soft,
+      t = world_group<4, MAXS, TG>(a, ob, Ms + Mc + Mb, a.w.Mh, gl, gm, ls, lsph + l * S, Tl, Bw, bl.w, want_soft,
                                    want_j, inv_tau, gref[4], csum);
       if (gl == 4) mine = t;
       // self group: the pairs listing link l; lane gl takes entries gl, gl + TG, ...
