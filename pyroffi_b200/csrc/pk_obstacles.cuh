@@ -375,43 +375,42 @@ __device__ __forceinline__ bool obstacle_near(const ObsView& ob, int m, float3 B
   return (B.x - h[3]) * h[0] + (B.y - h[4]) * h[1] + (B.z - h[5]) * h[2] - R < margin;
 }
 
-// Calls f(m, ObsKind<KIND>()) for each of the `count` obstacles base, base + 1,
-// ... of one kind that is in this lane's share (every stride-th from `lane`)
-// and that obstacle_near keeps, in increasing order.  The broad phase of up to
-// 32 obstacles goes into a survivor mask first, then f runs on the survivors:
-// the lanes of a warp hold different configurations and keep different
-// obstacles, so calling f from inside the test loop would run it once for
-// every obstacle that any lane keeps (about 60% of the trajectory workload's
-// 144 per lane and link) instead of max-over-lanes survivors times (about 9).
-// 512 x 64 x 7 trajectories among 288 obstacles, forward and backward
-// launches: 395 -> 336 us, the same bits.
-template <int KIND, class F>
-__device__ __forceinline__ void near_of_kind(const ObsView& ob, int base, int count, float3 B, float R, float margin,
+// Calls f(m, ObsKind<KIND>()) for each of the `count` obstacles index(0),
+// index(1), ... of one kind that is in this lane's share (every stride-th from
+// `lane`) and that obstacle_near keeps, in that order.  The broad phase of up
+// to 32 obstacles goes into a survivor mask first, then f runs on the
+// survivors: the lanes of a warp hold different configurations and keep
+// different obstacles, so calling f from inside the test loop would run it once
+// for every obstacle that any lane keeps (about 60% of the trajectory
+// workload's 144 per lane and link) instead of max-over-lanes survivors times
+// (about 9).  512 x 64 x 7 trajectories among 288 obstacles, forward and
+// backward launches: 395 -> 336 us, the same bits.
+template <int KIND, class Index, class F>
+__device__ __forceinline__ void near_of_kind(const ObsView& ob, Index index, int count, float3 B, float R, float margin,
                                              int lane, int stride, F& f) {
   for (int k0 = lane; k0 < count; k0 += 32 * stride) {
     unsigned mask = 0u;
     const int n = min(32, (count - k0 + stride - 1) / stride);
 #pragma unroll 4
     for (int i = 0; i < n; ++i)
-      if (obstacle_near<KIND>(ob, base + k0 + i * stride, B, R, margin)) mask |= 1u << i;
+      if (obstacle_near<KIND>(ob, index(k0 + i * stride), B, R, margin)) mask |= 1u << i;
     while (mask) {
       const int i = __ffs(mask) - 1;
       mask &= mask - 1u;
-      f(base + k0 + i * stride, ObsKind<KIND>());
+      f(index(k0 + i * stride), ObsKind<KIND>());
     }
   }
 }
 
-// Calls f(m, ObsKind<kind>()) for each obstacle m of this lane's share --
-// every stride-th obstacle of each kind from `lane` -- that obstacle_near
-// keeps: one pass per kind, so neither the test nor f needs to dispatch.
+// The same for all obstacles of the kinds other than spheres: one pass per
+// kind, so neither the test nor f needs to dispatch.
 template <class F>
-__device__ __forceinline__ void for_each_near_obstacle(const ObsView& ob, float3 B, float R, float margin, int lane,
-                                                       int stride, F&& f) {
-  near_of_kind<0>(ob, 0, ob.Ms, B, R, margin, lane, stride, f);
-  near_of_kind<1>(ob, ob.Ms, ob.Mc, B, R, margin, lane, stride, f);
-  near_of_kind<2>(ob, ob.Ms + ob.Mc, ob.Mb, B, R, margin, lane, stride, f);
-  near_of_kind<3>(ob, ob.Ms + ob.Mc + ob.Mb, ob.Mh, B, R, margin, lane, stride, f);
+__device__ __forceinline__ void for_each_near_other(const ObsView& ob, float3 B, float R, float margin, int lane,
+                                                    int stride, F&& f) {
+  const int b1 = ob.Ms, b2 = b1 + ob.Mc, b3 = b2 + ob.Mb;
+  near_of_kind<1>(ob, [=](int i) { return b1 + i; }, ob.Mc, B, R, margin, lane, stride, f);
+  near_of_kind<2>(ob, [=](int i) { return b2 + i; }, ob.Mb, B, R, margin, lane, stride, f);
+  near_of_kind<3>(ob, [=](int i) { return b3 + i; }, ob.Mh, B, R, margin, lane, stride, f);
 }
 
 __device__ __forceinline__ float3 cross3(float3 a, float3 b) {
@@ -425,6 +424,14 @@ __device__ __forceinline__ int float_to_ordered(float f) {
 }
 __device__ __forceinline__ float ordered_to_float(int i) {
   return __int_as_float((i >= 0) ? i : (i ^ 0x7fffffff));
+}
+
+// Minimum and maximum over the lanes of `mask` (their float order, NaN aside).
+__device__ __forceinline__ float warp_min_of(unsigned mask, float v) {
+  return ordered_to_float(__reduce_min_sync(mask, float_to_ordered(v)));
+}
+__device__ __forceinline__ float warp_max_of(unsigned mask, float v) {
+  return ordered_to_float(__reduce_max_sync(mask, float_to_ordered(v)));
 }
 
 __device__ __forceinline__ float warp_min(float v, unsigned mask = 0xffffffffu) {

@@ -248,7 +248,7 @@ __device__ __forceinline__ SoftAcc world_group(const ScoLinArgs& a, const ObsVie
       link_min(o, dmin, arg);
       csum -= colldist(dmin, a.margin);
     };
-    near_of_kind<KIND - 1>(ob, base, count, B, R, a.margin, gl, TG, add);
+    near_of_kind<KIND - 1>(ob, [=](int i) { return base + i; }, count, B, R, a.margin, gl, TG, add);
     return acc;
   }
   for (int k = gl; k < count; k += TG) {
