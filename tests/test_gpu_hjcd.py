@@ -88,6 +88,54 @@ def test_stop_flag_ends_every_seed_of_the_problem():
     np.testing.assert_allclose(err.cpu().numpy(), e0.cpu().numpy(), rtol=1e-6)
 
 
+def odd_robot(n_joints):
+    """A tree of revolute, prismatic, fixed and mimic joints, listed out of order (child before parent)."""
+    from pyroffi_b200.robot import RobotModel
+    rng = np.random.default_rng(n_joints)
+    n = n_joints
+    parent = np.array([2, 0, -1, 2, 3, 4, 5, 6, 3][:n])
+    kinds = ["rev", "rev", "pris", "fixed", "rev", "rev", "rev", "rev", "rev"][:n]
+    twists, ptf = np.zeros((n, 6)), np.zeros((n, 7))
+    act, mimic, mul, off = -np.ones(n, int), -np.ones(n, int), np.ones(n), np.zeros(n)
+    a = 0
+    for j, k in enumerate(kinds):
+        v = rng.normal(size=3)
+        twists[j, 0 if k == "pris" else 3:3 if k == "pris" else 6] = 0 if k == "fixed" else v / np.linalg.norm(v)
+        q = rng.normal(size=4)
+        ptf[j] = [*(q / np.linalg.norm(q)), *rng.uniform(-0.3, 0.3, 3)]
+        if k == "fixed":
+            continue
+        if j == 5:                                     # follows actuated joint 0
+            mimic[j], mul[j], off[j] = 0, -0.5, 0.1
+            continue
+        act[j] = a
+        a += 1
+    return RobotModel(twists=twists, parent_tf=ptf, parent_idx=parent, act_idx=act, mimic_mul=mul, mimic_off=off,
+                      mimic_act_idx=mimic, parent_joint_indices=np.arange(-1, n), lower=-1.5 * np.ones(a),
+                      upper=1.5 * np.ones(a))
+
+
+@pytest.mark.parametrize("n_joints", [1, 3, 5, 8, 9])
+@pytest.mark.parametrize("S", [1, 31, 33])
+def test_coarse_lanes_on_trees(n_joints, S):
+    """The eight-lane coarse kernel (up to 8 joints; 9 take the other one) against the FP64 oracle: trees,
+    prismatic, fixed and mimic joints, partial blocks.  A near-tie of two joints may go the other way."""
+    m = odd_robot(n_joints)
+    rng = np.random.default_rng(S)
+    link = m.n_links - 1
+    sol = HjcdSolver(m, link, device=DEV)
+    from oracle import kinematics as okin
+    tgt = okin.forward_kinematics(m.random_cfgs(rng, 2).astype(np.float64), m.as_dict())[:, link].astype(np.float32)
+    seeds = rng.uniform(m.lower, m.upper, size=(2, S, m.n_act)).astype(np.float32)
+    cfg, err = sol.coarse(t(seeds), t(tgt), k_max=6)
+    rates = []
+    for p in range(2):
+        ocfg, oe = ohjcd.coarse(seeds[p], tgt[p:p + 1, None], m.as_dict(), [m.link_joint(link)],
+                                [m.ancestor_mask(link)], m.lower, m.upper, np.zeros(m.n_act, bool), 6)
+        rates.append(agree(err[p].cpu().numpy(), oe, atol=1e-6))
+    assert np.mean(rates) >= 0.9, rates
+
+
 def test_fixed_joints_do_not_move():
     w, sol, *_ = chain(S=16)
     mask = np.zeros(w.model.n_act, np.int32)
