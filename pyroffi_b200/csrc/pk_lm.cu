@@ -17,8 +17,10 @@
 //    (cheap) FK / Jacobian / damped-step math redundantly, so the group's
 //    decisions are bit-identical without broadcasts; with TPS > 1 the
 //    (dominant) collision penalty is split over the group's lanes and the
-//    partial sums meet in a butterfly shuffle; with one lane per seed the
-//    self pairs are drained by the whole warp (self_warp).
+//    partial sums meet in a butterfly shuffle; with one lane per
+//    configuration the self pairs are drained by the whole warp (self_warp).
+//    By default the 8-wide kernel gives a seed two lanes that share out the
+//    line-search trials (trial lanes), each with a configuration of its own.
 //  * robot description, obstacle set, sphere list, limits and this block's
 //    targets are staged once per block in shared memory; joint poses of
 //    each lane live in a bank-strided shared slot array; configuration,
@@ -69,6 +71,7 @@ struct LmArgs {
   int coll;
   float coll_w, margin;
   int spb;
+  int trial_lanes;  // seed-group kernel, one lane per configuration: lanes per seed that share the line search
   int f64_solve;  // the damped step's system in FP64 (seed-group kernel, one lane per seed); else FP32
   int grid_n;     // obstacle grid cells per axis (0: no grid, every obstacle takes the bounding test)
   int grid_auto;  // grid_n is the default resolution (the launch may coarsen it; see lm_fit_grid)
@@ -115,7 +118,7 @@ __host__ __device__ __forceinline__ int lm_ms_pad(int Ms, int tps) {
 }
 
 // Self-pair groups per chunk of the warp item list (one lane per seed).
-constexpr int kSelfChunk = 16;
+constexpr int kSelfChunk = 4;
 
 // Seeds per block of the 16-wide one-lane kernel by default: the 16-DOF /
 // 2-EE register state takes the whole register file at 2 blocks of 128
@@ -129,17 +132,18 @@ __host__ __device__ __forceinline__ int lm_pos4_stride(int n_rs) { return n_rs +
 
 // Byte offsets of the LM block's dynamic shared memory.
 struct LmLayout {
-  size_t rs, rsp, ws, pairs, pair4, prec, pgstart, wscr, gjoint, gstart, rsj, rsk, cells, cell_obs, wc, wb, wh, slots, cen, pos, scratch,
+  size_t rs, rsp, ws, pairs, pair4, prec, pgstart, wscr, gjoint, gstart, rsj, rsk, cells, cell_obs, wc, wb, wh, slots, pos, scratch,
       total;
   int ms_pad, grid, max_entries, scratch_ints, recs;
 };
 
 __host__ __device__ inline size_t lm_align16(size_t x) { return (x + 15) & ~size_t(15); }
 
-// threads == 0: seed-group kernel.  Per seed, the joint pose slots and the
-// bounding-sphere centres, both laid out item-major ([item][spb]: component
-// c of item i of seed g at (i * K + c) * spb + g), so seeds reading the same
-// item hit distinct banks.  Sphere world positions are never stored: world
+// threads == 0: seed-group kernel.  Per configuration in flight (one per seed,
+// or one per trial lane), the joint pose slots and the bounding-sphere centres,
+// both laid out item-major ([item][nc]: component c of item i of configuration
+// g at (i * K + c) * nc + g), so lanes reading the same item hit distinct
+// banks.  Sphere world positions are never stored: world
 // obstacles are moved into joint frames and self pairs go through one
 // relative transform per joint pair.  Both run on packed FP32x2 arithmetic,
 // two spheres or two pairs per operation, from paired tables: each joint's
@@ -156,9 +160,11 @@ __host__ __device__ inline LmLayout lm_layout(const LmArgs& a, int tps, int thre
   LmLayout L;
   size_t o = lm_align16(sizeof(LmShared));
   const int n_rs = a.n_rs, n_self = a.coll ? a.n_self : 0;
+  const int nc = a.spb * max(a.trial_lanes, 1);  // configurations in flight
   L.ms_pad = lm_ms_pad(a.w.Ms, tps);
   if (threads == 0) {
-    L.scratch_ints = a.coll ? max(a.m.n_joints * a.m.n_joints, a.w.Ms) : 0;
+    // obstacle boxes and the grid's offsets as ints while it is built
+    L.scratch_ints = a.coll ? max(a.m.n_joints, a.w.Ms + 4 + obstacle_grid_cells(a.grid_n) + 1) : 0;
   } else {
     L.scratch_ints = 7 * a.m.n_joints * threads;  // the pose slots double as staging scratch
   }
@@ -179,19 +185,16 @@ __host__ __device__ inline LmLayout lm_layout(const LmArgs& a, int tps, int thre
   L.pgstart = o; o = lm_align16(o + (threads == 0 ? 4 * (size_t)(n_self + 2) : 0));
   // one lane per seed: per warp, the self-pair item list (kSelfChunk * 32 u16)
   // and the item sums (kSelfChunk * 32 floats)
-  L.wscr = o; o = lm_align16(o + ((threads == 0 && tps == 1 && n_self > 0) ? (size_t)(a.spb / 32) * kSelfChunk * 32 * 6 : 0));
+  L.wscr = o; o = lm_align16(o + ((threads == 0 && tps == 1 && n_self > 0) ? (size_t)(nc / 32) * kSelfChunk * 32 * 6 : 0));
   L.recs = threads == 0 ? 1 : 0;
   L.gjoint = o; o = lm_align16(o + 8 * (size_t)(n_self + 1));
   L.gstart = o; o = lm_align16(o + 4 * (size_t)(n_self + 2));
   L.rsj = o; o = lm_align16(o + 4 * (size_t)n_rs);
   L.rsk = o; o = lm_align16(o + 4 * (size_t)n_rs);
-  L.cells = o; o = lm_align16(o + (L.grid ? 4 * (size_t)(obstacle_grid_cells(a.grid_n) + 1) : 0));
+  L.cells = o; o = lm_align16(o + (L.grid ? (threads == 0 ? 2 : 4) * (size_t)(obstacle_grid_cells(a.grid_n) + 1) : 0));
   L.cell_obs = o; o = lm_align16(o + 2 * (size_t)L.max_entries);
   if (threads == 0) {
-    L.slots = o; o = lm_align16(o + 28 * (size_t)a.m.n_joints * a.spb);
-    // bounding centres are kept per seed only where other lanes read them:
-    // lanes sharing a seed (tps > 1) or the warp-shared self-pair items
-    L.cen = o; o = lm_align16(o + ((a.coll && (tps > 1 || n_self > 0)) ? 12 * (size_t)a.m.n_joints * a.spb : 0));
+    L.slots = o; o = lm_align16(o + 28 * (size_t)a.m.n_joints * nc);
     L.scratch = L.slots;
     L.pos = o;
     o = max(o, lm_align16(L.scratch + 4 * (size_t)L.scratch_ints));
@@ -199,7 +202,6 @@ __host__ __device__ inline LmLayout lm_layout(const LmArgs& a, int tps, int thre
     L.slots = o; o = lm_align16(o + 28 * (size_t)a.m.n_joints * threads);
     L.pos = o; o = lm_align16(o + 16 * (size_t)lm_pos4_stride(n_rs) * a.spb);
     L.scratch = L.slots;
-    L.cen = L.pos;
   }
   L.total = o;
   return L;
@@ -251,16 +253,20 @@ struct PenaltyCtx {
   const float4* prec;    // self pairs in pairs, 4 float4 per pair of pairs (the layout's paired pair table)
   const int2* gjoint;    // [n_groups] joint slots (x, y) of each self-pair group
   const int* pgstart;    // [n_groups + 1] padded pair range of each group (even)
-  const int* cell_start; // [G^3 + 1] obstacle grid (null: no grid, scan every obstacle)
+  const unsigned short* cell_start; // [G^3 + 1] obstacle grid (null: no grid, scan every obstacle)
   const unsigned short* cell_obs;
-  float* cen;            // this seed's bounding centres: component c of slot j at cen[(3 j + c) * cs]
-                         // (null: not kept; each lane computes its seed's centres where it needs them)
-  int cs;
   float3 glo, ginv;      // grid origin and inverse cell size
   int gn;                // grid cells per axis
   int n_rs, n_js, n_groups, Ms_pad, Mc, Mb, Mh;
   float margin;
 };
+
+// Bounding centre of joint slot j, once penalty_share has put it in place of
+// the joint's position.
+__device__ __forceinline__ float3 slot_centre(const PenaltyCtx& c, const PoseSlots& ps, int j) {
+  const float* p = ps.base + (c.jlist[j] * 7 + 4) * ps.stride;
+  return make_float3(p[0], p[ps.stride], p[2 * ps.stride]);
+}
 
 // Hinge term of a sphere pair given squared centre distance d2 and
 // rr = r_a + r_b + margin: (d - margin)^2 when d < margin.  Tested on d2
@@ -274,11 +280,12 @@ __device__ __forceinline__ void hinge_sq(float d2, float rr, float& pen) {
 
 // Exact hinge terms of the sphere pairs [p0, p1) of a joint against world
 // sphere O (radius already + margin), with the obstacle centre moved into
-// the joint's frame (T) once: |R c_k + t - o| = |c_k - R^T (o - t)|; two
+// the joint's frame (T: the joint's rotation and its bounding centre, jb) once: |R c_k + t - o| = |c_k - R^T (o - t)|; two
 // spheres per packed FP32x2 operation, terms added in sphere order.
-__device__ __forceinline__ void narrow_world(const PenaltyCtx& c, const Pose& T, int p0, int p1, float4 O,
+__device__ __forceinline__ void narrow_world(const PenaltyCtx& c, const Pose& T, float4 jb, int p0, int p1, float4 O,
                                              float& pen) {
-  const float3 o = pose_apply_inv(T, make_float3(O.x, O.y, O.z));
+  float3 o = pose_apply_inv(T, make_float3(O.x, O.y, O.z));  // relative to the bounding centre
+  o.x += jb.x; o.y += jb.y; o.z += jb.z;
   const float2 nx = make_float2(-o.x, -o.x), ny = make_float2(-o.y, -o.y), nz = make_float2(-o.z, -o.z);
   const float2 ow = make_float2(O.w, O.w);
   for (int p = p0; p < p1; ++p) {
@@ -308,7 +315,9 @@ __device__ __forceinline__ void group_pairs(const PenaltyCtx& c, const PoseSlots
   const float qx = A.w * Bp.x - A.x * Bp.w - A.y * Bp.z + A.z * Bp.y;
   const float qy = A.w * Bp.y + A.x * Bp.z - A.y * Bp.w - A.z * Bp.x;
   const float qz = A.w * Bp.z - A.x * Bp.y + A.y * Bp.x - A.z * Bp.w;
-  const float3 u = pose_apply_inv(A, make_float3(Bp.tx, Bp.ty, Bp.tz));
+  // the slots hold bounding centres: t = B - R c, so u = R_x^T (B_y - B_x) + c_x - M c_y
+  float3 u = pose_apply_inv(A, make_float3(Bp.tx, Bp.ty, Bp.tz));
+  const float4 cx = c.jb[ja.x], cy = c.jb[ja.y];
   auto dup = [](float v) { return make_float2(v, v); };
   const float2 m00 = dup(1.f - 2.f * (qy * qy + qz * qz)), m01 = dup(2.f * (qx * qy - qw * qz)),
                m02 = dup(2.f * (qx * qz + qw * qy));
@@ -316,6 +325,9 @@ __device__ __forceinline__ void group_pairs(const PenaltyCtx& c, const PoseSlots
                m12 = dup(2.f * (qy * qz - qw * qx));
   const float2 m20 = dup(2.f * (qx * qz - qw * qy)), m21 = dup(2.f * (qy * qz + qw * qx)),
                m22 = dup(1.f - 2.f * (qx * qx + qy * qy));
+  u.x += cx.x - (m00.x * cy.x + m01.x * cy.y + m02.x * cy.z);
+  u.y += cx.y - (m10.x * cy.x + m11.x * cy.y + m12.x * cy.z);
+  u.z += cx.z - (m20.x * cy.x + m21.x * cy.y + m22.x * cy.z);
   const float2 ux = dup(u.x), uy = dup(u.y), uz = dup(u.z);
   // two pairs per packed FP32x2 operation: e = M c_b + u - c_a
   const int q1 = c.pgstart[gi + 1];
@@ -339,16 +351,13 @@ __device__ __forceinline__ void group_pairs(const PenaltyCtx& c, const PoseSlots
 // pairs of those groups in increasing group order.
 template <int TPS>
 __device__ __forceinline__ void self_share(const PenaltyCtx& c, const PoseSlots& ps, int t, float& pen) {
-  const float* const cen = c.cen;
-  const int cs = c.cs;
   int turn = 0;  // surviving groups seen so far (the same count on every lane of the seed)
   for (int g0 = 0; g0 < c.n_groups; g0 += 32) {
     unsigned mask = 0u;
     for (int i = 0; i < 32 && g0 + i < c.n_groups; ++i) {
       const int2 ja = c.gjoint[g0 + i];
-      const float dx = cen[(3 * ja.x) * cs] - cen[(3 * ja.y) * cs];
-      const float dy = cen[(3 * ja.x + 1) * cs] - cen[(3 * ja.y + 1) * cs];
-      const float dz = cen[(3 * ja.x + 2) * cs] - cen[(3 * ja.y + 2) * cs];
+      const float3 Bx = slot_centre(c, ps, ja.x), By = slot_centre(c, ps, ja.y);
+      const float dx = Bx.x - By.x, dy = Bx.y - By.y, dz = Bx.z - By.z;
       const float rr = c.jb[ja.x].w + c.jb[ja.y].w + c.margin;
       if (!(dx * dx + dy * dy + dz * dz < rr * fabsf(rr))) continue;
       if ((turn++ & (TPS - 1)) == t) mask |= 1u << i;
@@ -361,51 +370,36 @@ __device__ __forceinline__ void self_share(const PenaltyCtx& c, const PoseSlots&
   }
 }
 
-// Self pairs of the 32 seeds of a warp (TPS == 1), all 32 lanes together.
-// Per chunk of kSelfChunk groups, each lane culls the groups for its own
-// seed (none when !need); the surviving (seed, group) items go into the
-// warp's list in (group, lane) order; lane l takes items l, l + 32, ... and
-// writes each item's sum (its pairs in pair order) to res[group][seed]; then
-// each lane adds its own surviving groups' sums in group order.  The result
-// does not depend on which lane took which item, and the work of a chunk is
-// spread over the warp instead of following the seed with the most
-// surviving groups.  slots_w: the pose slots of the warp's first seed; b4:
-// the culls four groups per step.
-__device__ __forceinline__ void self_warp(const PenaltyCtx& c, float* slots_w, int spb, bool need, bool b4,
+// Self pairs of the 32 configurations of a warp (TPS == 1), all 32 lanes
+// together.  Per chunk of kSelfChunk groups, each lane culls the groups for
+// its own configuration (none when !need); the surviving (lane, group) items
+// go into the warp's list in (group, lane) order; lane l takes items l, l +
+// 32, ... and writes each item's sum (its pairs in pair order) to
+// res[group][lane]; then each lane adds its own surviving groups' sums in
+// group order.  The result does not depend on which lane took which item, and
+// the work of a chunk is spread over the warp instead of following the lane
+// with the most surviving groups.  slots_w: the pose slots of the warp's first
+// configuration.  The culls' loads are issued four groups at a time.
+__device__ __forceinline__ void self_warp(const PenaltyCtx& c, const PoseSlots& ps, float* slots_w, int spb, bool need,
                                           float& pen, unsigned short* list, float* res) {
   const int lane = threadIdx.x & 31;
-  const float* const cen = c.cen;
-  const int cs = c.cs;
   for (int g0 = 0; g0 < c.n_groups; g0 += kSelfChunk) {
     const int nc = min(kSelfChunk, c.n_groups - g0);
     unsigned mine = 0u;
     int n_items = 0;
-    // this lane's surviving groups of the chunk (B4: four groups' loads at a time)
-    if (need && !b4) {
-      for (int i = 0; i < nc; ++i) {
-        const int2 ja = c.gjoint[g0 + i];
-        const float dx = cen[(3 * ja.x) * cs] - cen[(3 * ja.y) * cs];
-        const float dy = cen[(3 * ja.x + 1) * cs] - cen[(3 * ja.y + 1) * cs];
-        const float dz = cen[(3 * ja.x + 2) * cs] - cen[(3 * ja.y + 2) * cs];
-        const float rr = c.jb[ja.x].w + c.jb[ja.y].w + c.margin;
-        if (dx * dx + dy * dy + dz * dz < rr * fabsf(rr)) mine |= 1u << i;
-      }
-    } else if (need) {
-      for (int i0 = 0; i0 < nc; i0 += 4) {
-        float d2[4], rr[4];
+    if (need) {
+      float d2[kSelfChunk], rr[kSelfChunk];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int2 ja = c.gjoint[g0 + min(i0 + u, nc - 1)];
-          const float dx = cen[(3 * ja.x) * cs] - cen[(3 * ja.y) * cs];
-          const float dy = cen[(3 * ja.x + 1) * cs] - cen[(3 * ja.y + 1) * cs];
-          const float dz = cen[(3 * ja.x + 2) * cs] - cen[(3 * ja.y + 2) * cs];
-          rr[u] = c.jb[ja.x].w + c.jb[ja.y].w + c.margin;
-          d2[u] = dx * dx + dy * dy + dz * dz;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (i0 + u < nc && d2[u] < rr[u] * fabsf(rr[u])) mine |= 1u << (i0 + u);
+      for (int u = 0; u < kSelfChunk; ++u) {
+        const int2 ja = c.gjoint[g0 + min(u, nc - 1)];
+        const float3 Bx = slot_centre(c, ps, ja.x), By = slot_centre(c, ps, ja.y);
+        const float dx = Bx.x - By.x, dy = Bx.y - By.y, dz = Bx.z - By.z;
+        rr[u] = c.jb[ja.x].w + c.jb[ja.y].w + c.margin;
+        d2[u] = dx * dx + dy * dy + dz * dz;
       }
+#pragma unroll
+      for (int u = 0; u < kSelfChunk; ++u)
+        if (u < nc && d2[u] < rr[u] * fabsf(rr[u])) mine |= 1u << u;
     }
     for (int i = 0; i < nc; ++i) {
       const bool sv = (mine >> i) & 1u;
@@ -433,7 +427,8 @@ __device__ __forceinline__ void self_warp(const PenaltyCtx& c, float* slots_w, i
 
 // Partial hinge penalty of lane t of a TPS-group (not weighted, not summed).
 //  1. lane t puts the bounding-sphere centres of joint slots t, t+TPS, ...
-//     (world frame) into this seed's shared slots;
+//     (world frame) into this configuration's pose slots, in place of the
+//     joints' positions (nothing after the penalty reads those);
 //  2. world spheres: conservative culls before any sphere-level test.  The
 //     joint's bounding sphere (centre B, radius R) can only reach obstacle o
 //     if |B - o| < R + r_o + margin.  With the obstacle grid, only the
@@ -468,29 +463,21 @@ template <int TPS, bool B4>
 __device__ float penalty_share(const PenaltyCtx& c, const PoseSlots& ps, int t, unsigned gmask, bool need,
                                float* slots_w, int spb, unsigned short* wlist, float* wres) {
   float pen = 0.f;
-  float* const cen = c.cen;
-  const int cs = c.cs;
   const bool b4 = B4;
-  // bounding centre of joint slot j: kept per seed, or computed here
-  auto centre = [&](int j) {
-    if (cen) return make_float3(cen[(3 * j) * cs], cen[(3 * j + 1) * cs], cen[(3 * j + 2) * cs]);
-    const float4 bl = c.jb[j];
-    return pose_apply(ps.load(c.jlist[j]), make_float3(bl.x, bl.y, bl.z));
-  };
   if (need) {
-    if (cen) {
-      for (int j = t; j < c.n_js; j += TPS) {
-        const Pose T = ps.load(c.jlist[j]);
-        const float4 bl = c.jb[j];
-        const float3 B = pose_apply(T, make_float3(bl.x, bl.y, bl.z));
-        cen[(3 * j) * cs] = B.x; cen[(3 * j + 1) * cs] = B.y; cen[(3 * j + 2) * cs] = B.z;
-      }
-      if (TPS > 1) __syncwarp(gmask);
+    for (int j = t; j < c.n_js; j += TPS) {
+      const int js = c.jlist[j];
+      const float4 bl = c.jb[j];
+      const float3 B = pose_apply(ps.load(js), make_float3(bl.x, bl.y, bl.z));
+      float* p = ps.base + (js * 7 + 4) * ps.stride;
+      p[0] = B.x; p[ps.stride] = B.y; p[2 * ps.stride] = B.z;
     }
+    if (TPS > 1) __syncwarp(gmask);
 
     for (int j = 0; j < c.n_js && c.Ms_pad > 0; ++j) {
-      const float R = c.jb[j].w;
-      const float3 Bj = centre(j);
+      const float4 jb = c.jb[j];
+      const float R = jb.w;
+      const float3 Bj = slot_centre(c, ps, j);
       const float Bx = Bj.x, By = Bj.y, Bz = Bj.z;
       const int p0 = c.pjstart[j], p1 = c.pjstart[j + 1];
       if (c.cell_start) {
@@ -540,7 +527,7 @@ __device__ float penalty_share(const PenaltyCtx& c, const PoseSlots& ps, int t, 
             while (mask) {
               const int i = __ffs(mask) - 1;
               mask &= mask - 1u;
-              narrow_world(c, T, p0, p1, c.ws[c.cell_obs[e0 + i * TPS]], pen);
+              narrow_world(c, T, jb, p0, p1, c.ws[c.cell_obs[e0 + i * TPS]], pen);
             }
           }
         }
@@ -559,7 +546,7 @@ __device__ float penalty_share(const PenaltyCtx& c, const PoseSlots& ps, int t, 
             while (mask) {
               const int i = __ffs(mask) - 1;
               mask &= mask - 1u;
-              narrow_world(c, T, p0, p1, c.ws[ob + i * TPS], pen);
+              narrow_world(c, T, jb, p0, p1, c.ws[ob + i * TPS], pen);
             }
           }
         }
@@ -568,10 +555,13 @@ __device__ float penalty_share(const PenaltyCtx& c, const PoseSlots& ps, int t, 
 
     if (c.Mc + c.Mb + c.Mh > 0) {
       for (int j = t; j < c.n_js; j += TPS) {
-        const float3 B = centre(j);
-        const float R = c.jb[j].w;
+        const float3 B = slot_centre(c, ps, j);
+        const float4 jb = c.jb[j];
+        const float R = jb.w;
         const int k0 = c.jstart[j], k1 = c.jstart[j + 1];
-        const Pose T = ps.load(c.jlist[j]);
+        Pose T = ps.load(c.jlist[j]);
+        const float3 off = quat_rotate(T.w, T.x, T.y, T.z, make_float3(jb.x, jb.y, jb.z));
+        T.tx -= off.x; T.ty -= off.y; T.tz -= off.z;  // the joint's position again
         for (int m = 0; m < c.Mc; ++m) {
           if (!(d_sphere_capsule(B, R, c.wc + 7 * m) < c.margin)) continue;
           for (int k = k0; k < k1; ++k) {
@@ -600,7 +590,10 @@ __device__ float penalty_share(const PenaltyCtx& c, const PoseSlots& ps, int t, 
 
     if (TPS > 1) self_share<TPS>(c, ps, t, pen);
   }
-  if (TPS == 1 && c.n_groups > 0) self_warp(c, slots_w, spb, need, b4, pen, wlist, wres);
+  if (TPS == 1 && c.n_groups > 0) {
+    __syncwarp();  // other lanes read this lane's slots
+    self_warp(c, ps, slots_w, spb, need, pen, wlist, wres);
+  }
   __syncwarp(gmask);
   return pen;
 }
@@ -1148,10 +1141,11 @@ __device__ void lm_stage(const LmArgs& a, unsigned char* smem_raw, const LmLayou
     __syncthreads();
   }
 
+  int* cell_int = L.recs ? scratch + ((a.w.Ms + 3) & ~3) : cell_start;
   if (sh.grid_on) {
     if (tid < 32) obstacle_grid_bounds(ws4, a.w.Ms, sh.rmax, a.grid_n, sh.glo, sh.ginv);
     __syncthreads();
-    obstacle_grid_build(ws4, a.w.Ms, sh.rmax, sh.grid_n, sh.glo, sh.ginv, scratch, cell_start, cell_obs,
+    obstacle_grid_build(ws4, a.w.Ms, sh.rmax, sh.grid_n, sh.glo, sh.ginv, scratch, cell_int, cell_obs,
                         L.max_entries, sh.grid_on);
     // a fine grid whose lists overflow the capacity falls back to the default
     // resolution (fewer, longer lists) before going without a grid
@@ -1163,8 +1157,14 @@ __device__ void lm_stage(const LmArgs& a, unsigned char* smem_raw, const LmLayou
         sh.grid_on = 1;
       }
       __syncthreads();
-      obstacle_grid_build(ws4, a.w.Ms, sh.rmax, sh.grid_n, sh.glo, sh.ginv, scratch, cell_start, cell_obs,
+      obstacle_grid_build(ws4, a.w.Ms, sh.rmax, sh.grid_n, sh.glo, sh.ginv, scratch, cell_int, cell_obs,
                           L.max_entries, sh.grid_on);
+    }
+    if (L.recs) {
+      // the seed-group kernels keep the offsets (at most 16,384) in 16 bits
+      unsigned short* cell16 = reinterpret_cast<unsigned short*>(cell_start);
+      for (int c = tid; c <= obstacle_grid_cells(sh.grid_n); c += nth) cell16[c] = (unsigned short)cell_int[c];
+      __syncthreads();
     }
   }
 }
@@ -1176,24 +1176,27 @@ __device__ void lm_stage(const LmArgs& a, unsigned char* smem_raw, const LmLayou
 // past `count`, which reads and writes nothing): a done seed's lanes run
 // along without changing its state, so the warp's collective steps
 // (self_warp) always see all 32 lanes.  No block-wide barrier.
-template <int MAXA, int MAXEE, int TPS, bool F64S = false, bool B4 = false>
+template <int MAXA, int MAXEE, int TPS, bool F64S = false, bool B4 = false, int TL = 1>
 __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* smem_raw, const LmLayout& L, int pb,
                                                int count, size_t gs_base) {
   LmShared& sh = *reinterpret_cast<LmShared*>(smem_raw);
   float4* rs4 = reinterpret_cast<float4*>(smem_raw + L.rs);
   float4* ws4 = reinterpret_cast<float4*>(smem_raw + L.ws);
   int2* gjoint = reinterpret_cast<int2*>(smem_raw + L.gjoint);
-  int* gstart = reinterpret_cast<int*>(smem_raw + L.gstart);
   int* cell_start = reinterpret_cast<int*>(smem_raw + L.cells);
   unsigned short* cell_obs = reinterpret_cast<unsigned short*>(smem_raw + L.cell_obs);
   float* wc = reinterpret_cast<float*>(smem_raw + L.wc);
   float* wb = reinterpret_cast<float*>(smem_raw + L.wb);
   float* wh = reinterpret_cast<float*>(smem_raw + L.wh);
   float* slots = reinterpret_cast<float*>(smem_raw + L.slots);
-  float* cen = reinterpret_cast<float*>(smem_raw + L.cen);
   const float4* prec = reinterpret_cast<const float4*>(smem_raw + L.prec);
+  static_assert(TL == 1 || TPS == 1, "trial lanes: one lane per configuration");
+  constexpr int SL = TPS * TL;  // lanes per seed
   const int tid = threadIdx.x;
-  const int g = tid / TPS, t = tid - g * TPS;
+  // seed g; t: lane within the lanes that split one configuration (TPS); tl:
+  // trial lane; cf: configuration in flight
+  const int g = tid / SL, t = TL > 1 ? 0 : tid - g * TPS, tl = TL > 1 ? tid - g * TL : 0;
+  const int cf = TL > 1 ? tid : g, ncf = TL > 1 ? a.spb * TL : a.spb;
   const int lane = tid & 31;
   const unsigned gmask = (TPS == 32) ? 0xffffffffu : (((1u << TPS) - 1u) << (lane & ~(TPS - 1)));
   const bool valid = g < count;
@@ -1202,7 +1205,7 @@ __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* s
 
   const JointTable& jt = sh.jt;
   // one pose-slot set per seed (written by lane 0 of the group, read by all)
-  const PoseSlots ps{slots + g, a.spb};
+  const PoseSlots ps{slots + cf, ncf};
   const bool leader = (t == 0);
   const bool use_coll = a.coll && (sh.n_rs > 0);
   PenaltyCtx pc;
@@ -1210,8 +1213,8 @@ __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* s
   pc.rsp = reinterpret_cast<const float4*>(smem_raw + L.rsp); pc.pjstart = sh.pjstart;
   pc.ws = ws4; pc.wc = wc; pc.wb = wb; pc.wh = wh; pc.prec = prec; pc.gjoint = gjoint;
   pc.pgstart = reinterpret_cast<const int*>(smem_raw + L.pgstart);
-  pc.cell_start = sh.grid_on ? cell_start : nullptr; pc.cell_obs = cell_obs;
-  pc.cen = (TPS > 1 || (a.coll && a.n_self > 0)) ? cen + g : nullptr; pc.cs = a.spb; pc.glo = sh.glo; pc.ginv = sh.ginv; pc.gn = sh.grid_n;
+  pc.cell_start = sh.grid_on ? reinterpret_cast<const unsigned short*>(cell_start) : nullptr; pc.cell_obs = cell_obs;
+  pc.glo = sh.glo; pc.ginv = sh.ginv; pc.gn = sh.grid_n;
   pc.n_rs = sh.n_rs; pc.n_js = sh.n_js; pc.n_groups = sh.n_groups; pc.Ms_pad = L.ms_pad;
   pc.Mc = a.w.Mc; pc.Mb = a.w.Mb; pc.Mh = a.w.Mh; pc.margin = a.margin;
 
@@ -1223,7 +1226,7 @@ __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* s
     cfg[i] = (valid && i < a.n_act) ? a.seeds[gs * a.n_act + i] : 0.f;
     best[i] = cfg[i];
   }
-  float* const slots_w = slots + (g & ~31);  // one lane per seed: the pose slots of the warp's first seed
+  float* const slots_w = slots + (cf & ~31);  // one lane per configuration: the pose slots of the warp's first one
   unsigned short* const wlist =
       reinterpret_cast<unsigned short*>(smem_raw + L.wscr) + (size_t)(tid >> 5) * kSelfChunk * 32 * 3;
   float* const wres = reinterpret_cast<float*>(wlist + kSelfChunk * 32);
@@ -1233,7 +1236,7 @@ __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* s
   auto penalty = [&](bool need) -> float {
     if (!use_coll) return 0.f;
     if (TPS > 1 && !need) return 0.f;
-    const float share = penalty_share<TPS, B4>(pc, ps, t, gmask, need, slots_w, a.spb, wlist, wres);
+    const float share = penalty_share<TPS, B4>(pc, ps, t, gmask, need, slots_w, ncf, wlist, wres);
     return a.coll_w * group_sum<TPS>(share, gmask);
   };
   // Every lane of the group computes the FK (same values); lane 0 stores it.
@@ -1254,9 +1257,10 @@ __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* s
   };
 
   // Evaluation schedule: ev = -1 the initial point, then per iteration ev = 0
-  // (current point: residual, Jacobian, damped step) and ev = 1..5 (the
-  // line-search trials).  A single call site each for FK, residual and
-  // penalty keeps the kernel small enough for the instruction cache.
+  // (current point: residual, Jacobian, damped step) and the 5 line-search
+  // trials, TL at a time (ev = 1, 1 + TL, ...: trial lane tl takes trial ev - 1
+  // + tl).  A single call site each for FK, residual and penalty keeps the
+  // kernel small enough for the instruction cache.
   float r[6 * MAXEE], pee[3 * MAXEE];
   float delta[MAXA];
   float lam = a.lam0;
@@ -1271,9 +1275,11 @@ __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* s
   // a seed's state from changing
   while (!__all_sync(0xffffffffu, done)) {
     float q[MAXA];
+    const int trial_i = ev - 1 + tl;  // this lane's trial (5 and up: none, it repeats the last)
+    const float alpha_i = line_alpha(min(trial_i, 4));
 #pragma unroll
     for (int c = 0; c < MAXA; ++c)
-      q[c] = (ev <= 0) ? cfg[c] : fmaxf(sh.lo[c], fminf(sh.hi[c], cfg[c] + line_alpha(ev - 1) * delta[c]));
+      q[c] = (ev <= 0) ? cfg[c] : fmaxf(sh.lo[c], fminf(sh.hi[c], cfg[c] + alpha_i * delta[c]));
     run_fk(q);
     ee_residual<MAXEE>(sh, ps, a.n_ee, r, pee);
 
@@ -1294,6 +1300,7 @@ __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* s
         if (all_conv) {
           done = true;
         } else {
+          // the lanes of a seed hold the same state and compute the same step
           curr = lm_direction<MAXA, MAXEE, F64S>(sh, ps, a.n_ee, W, r, pee, lam, max_p, max_o, delta) + pen_cur;
           best_a_err = 1e30f;
           best_a_pen = pen_cur;
@@ -1307,44 +1314,65 @@ __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* s
     // The penalty is >= 0, so a trial whose pose error alone is not below
     // the best trial so far cannot win (wsq + pen >= wsq in FP32 too): its
     // penalty is skipped, which leaves every decision and output unchanged.
-    // (The test is uniform across the seed's lanes.)
+    // (The test is uniform across the lanes that split a configuration.)
     const float wsq = weighted_sq(r);
-    const float pen = penalty(!done && (ev < 0 || wsq < best_a_err));
-    if (!done) {
-      const float err = wsq + pen;
-      if (ev < 0) {
-        pen_cur = pen;
-        best_err = err;
+    const bool mine = ev < 0 ? tl == 0 : trial_i < 5;
+    const float pen = penalty(!done && mine && (ev < 0 || wsq < best_a_err));
+    const float err = wsq + pen;
+    if (ev < 0) {
+      const float p0 = TL > 1 ? __shfl_sync(0xffffffffu, pen, lane & ~(TL - 1)) : pen;
+      const float e0 = TL > 1 ? __shfl_sync(0xffffffffu, err, lane & ~(TL - 1)) : err;
+      if (!done) {
+        pen_cur = p0;
+        best_err = e0;
         if (a.max_iter <= 0) done = true;
-      } else {
-        if (err < best_a_err) { best_a_err = err; best_a = ev - 1; best_a_pen = pen; }
-        if (ev == 5) {
-          // accept / reject the damped step, track the all-time best
-          const float alpha = line_alpha(best_a);
-          float trial[MAXA];
-#pragma unroll
-          for (int c = 0; c < MAXA; ++c) trial[c] = fmaxf(sh.lo[c], fminf(sh.hi[c], cfg[c] + alpha * delta[c]));
-          if (best_a_err < curr * (1.0f - 1e-4f)) {
-#pragma unroll
-            for (int c = 0; c < MAXA; ++c) cfg[c] = trial[c];
-            pen_cur = best_a_pen;
-            lam = fmaxf(lam * a.lam_down, 1e-10f);
-          } else {
-            lam = fminf(lam * a.lam_up, 1e6f);
-          }
-          if (best_a_err < best_err) {
-            best_err = best_a_err;
-#pragma unroll
-            for (int c = 0; c < MAXA; ++c) best[c] = trial[c];
-          }
-          if (++it >= a.max_iter) done = true;
-        }
       }
+      ev = 0;
+      continue;
     }
-    ev = (ev < 0 || ev == 5) ? 0 : ev + 1;
+    if (TL > 1) {
+      // the trials of this round in order, the first minimum wins; a skipped
+      // trial's error is its pose error alone, not below the best already
+#pragma unroll
+      for (int k = 0; k < TL; ++k) {
+        const float ek = __shfl_sync(0xffffffffu, err, (lane & ~(TL - 1)) + k);
+        const float pk = __shfl_sync(0xffffffffu, pen, (lane & ~(TL - 1)) + k);
+        if (!done && ev - 1 + k < 5 && ek < best_a_err) { best_a_err = ek; best_a = ev - 1 + k; best_a_pen = pk; }
+      }
+    } else if (!done && err < best_a_err) {
+      best_a_err = err;
+      best_a = ev - 1;
+      best_a_pen = pen;
+    }
+    if (ev + TL <= 5) {
+      ev += TL;
+      continue;
+    }
+    if (!done) {
+      // accept / reject the damped step, track the all-time best
+      const float alpha = line_alpha(best_a);
+      float trial[MAXA];
+#pragma unroll
+      for (int c = 0; c < MAXA; ++c) trial[c] = fmaxf(sh.lo[c], fminf(sh.hi[c], cfg[c] + alpha * delta[c]));
+      if (best_a_err < curr * (1.0f - 1e-4f)) {
+#pragma unroll
+        for (int c = 0; c < MAXA; ++c) cfg[c] = trial[c];
+        pen_cur = best_a_pen;
+        lam = fmaxf(lam * a.lam_down, 1e-10f);
+      } else {
+        lam = fminf(lam * a.lam_up, 1e6f);
+      }
+      if (best_a_err < best_err) {
+        best_err = best_a_err;
+#pragma unroll
+        for (int c = 0; c < MAXA; ++c) best[c] = trial[c];
+      }
+      if (++it >= a.max_iter) done = true;
+    }
+    ev = 0;
   }
 
-  if (t == 0 && valid) {
+  if (t == 0 && tl == 0 && valid) {
 #pragma unroll
     for (int c = 0; c < MAXA; ++c)
       if (c < a.n_act) a.out_cfg[gs * a.n_act + c] = best[c];
@@ -1356,15 +1384,15 @@ __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* s
 // thread at 128 registers (a few hundred bytes of spills at MAXA = 8); 2
 // leaves room for the whole seed state, for launches whose shared memory
 // admits only 2 blocks per SM anyway.
-template <int MAXA, int MAXEE, int TPS, int MINB, bool F64S = false, bool B4 = false>
-__global__ void __launch_bounds__(128, MINB) lm_kernel(LmArgs a) {
+template <int MAXA, int MAXEE, int TPS, int MINB, bool F64S = false, bool B4 = false, int TL = 1>
+__global__ void __launch_bounds__(128 * TL, MINB) lm_kernel(LmArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const LmLayout L = lm_layout(a, TPS);
   const int pb = blockIdx.y;
   lm_stage<MAXA>(a, smem_raw, L, pb);
   const int s_first = blockIdx.x * a.spb;
   const int count = min(a.spb, a.Sd - s_first);
-  lm_seed_groups<MAXA, MAXEE, TPS, F64S, B4>(a, smem_raw, L, pb, count, (size_t)pb * a.Sd + s_first);
+  lm_seed_groups<MAXA, MAXEE, TPS, F64S, B4, TL>(a, smem_raw, L, pb, count, (size_t)pb * a.Sd + s_first);
 }
 
 // Persistent seed-group kernel of pk_ik_batch: blocks take items (class,
@@ -1870,9 +1898,33 @@ static void lm_fit_grid(LmArgs& a, int tps, int threads = 0) {
     a.grid_n = kObsGridDefault;
 }
 
+// Two trial lanes per seed (the 8-wide one-lane kernel) where two of their
+// 256-thread blocks fit an SM: twice the warps, each with 3 rounds of trials
+// per iteration instead of 5.  One lane per seed leaves 1.7 warps per scheduler
+// on the IK benchmark's 32,768 seeds, each issuing every sixth cycle.
+// 256 problems x 128 seeds, 6 iterations: 1471 -> 1320 us (128 registers
+// instead of 248, so about 850 bytes of spills, in the step).  Not in the
+// batch's persistent kernel: 512 mixed problems 5575 us without, 5920 with.
+constexpr size_t kTwoTrialLanesSmem = (228 / 2 - 1) * 1024;
+
 template <int MAXA, int MAXEE, int TPS, bool F64S = false>
 static int launch_lm_t(const LmArgs& a0, cudaStream_t st) {
   LmArgs a = a0;
+  if constexpr (MAXA <= 8 && TPS == 1 && !F64S) {
+    if (a.trial_lanes == 2) {
+      lm_fit_grid(a, 1);
+      const size_t smem = lm_smem_bytes(a, 1);
+      if (smem <= kTwoTrialLanesSmem) {
+        auto kern = (a.coll && a.grid_n >= kObsGridFine) ? lm_kernel<MAXA, MAXEE, 1, 2, false, true, 2>
+                                                         : lm_kernel<MAXA, MAXEE, 1, 2, false, false, 2>;
+        if (int s = set_smem_limit((const void*)kern, smem)) return s;
+        kern<<<dim3((a.Sd + a.spb - 1) / a.spb, a.P), a.spb * 2, smem, st>>>(a);
+        return cuda_status(cudaGetLastError(), "lm_kernel launch");
+      }
+      a = a0;
+    }
+  }
+  a.trial_lanes = 1;
   lm_fit_grid(a, TPS);
   const int threads = a.spb * TPS;
   const size_t smem = lm_smem_bytes(a, TPS);
@@ -1946,7 +1998,11 @@ static int launch_lm(LmArgs a, int tps, int spb, cudaStream_t st) {
   // body, are routed by lm_common.)
   if (tps <= 0) {
     tps = 1;
-    if (spb <= 0) spb = (a.n_act <= 8 && a.n_ee <= 1) ? 128 : kSeedsPerBlock16;
+    if (spb <= 0) {
+      const bool small = a.n_act <= 8 && a.n_ee <= 1;
+      spb = small ? 128 : kSeedsPerBlock16;
+      a.trial_lanes = small && !a.f64_solve ? 2 : 1;
+    }
   }
   if (tps == 5) {
     PK_CHECK_ARG(!a.f64_solve, "fp64_solve runs with threads_per_seed 0 or 1");
@@ -2210,6 +2266,7 @@ static int launch_seed_group_body(const BatchCall& b, int body, cudaStream_t st,
     a.coll = o.enable_collision ? 1 : 0; a.coll_w = o.collision_weight; a.margin = o.collision_margin;
     if (!a.coll) a.n_self = 0;
     a.spb = spb;
+    a.trial_lanes = 1;
     a.grid_n = lm_grid_option(o.obstacle_grid, a.w.Ms);
     a.grid_auto = o.obstacle_grid == 0;
     if (int s = validate_lm(a)) return s;

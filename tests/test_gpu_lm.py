@@ -335,3 +335,20 @@ def test_lm_ragged_seed_counts():
     assert np.isfinite(errs.cpu().numpy()).all()
     close = np.abs(errs[1].cpu().numpy() - oe) <= 1e-3 * np.abs(oe) + 1e-4
     assert close.mean() >= 0.9
+
+
+@pytest.mark.parametrize("Sd", [1, 31, 129])
+@pytest.mark.parametrize("n_self", [0, 7, 200])
+@pytest.mark.parametrize("iters", [0, 3])
+def test_trial_lanes_equal_one_lane(Sd, n_self, iters):
+    """Two trial lanes per seed (the default mapping) against one lane per seed (asked for by
+    seeds_per_block): the same evaluations, so the same results but for roundings that the compiler
+    places differently in the two kernels."""
+    w = W.ik(P=3, Sd=Sd, n_self=n_self)
+    kw = dict(spheres=w.spheres, world=w.world, self_pairs=w.self_pairs, max_iter=iters, lambda_init=w.lambda_init,
+              lambda_down=w.lambda_down, lambda_up=w.lambda_up, device=DEV)
+    a = BatchIkSolver(w.model, w.target_link, **kw).run_lm(tt(w.target_T), tt(w.seeds))
+    b = BatchIkSolver(w.model, w.target_link, threads_per_seed=1, seeds_per_block=128, **kw).run_lm(tt(w.target_T),
+                                                                                                   tt(w.seeds))
+    close = ((a[0] - b[0]).abs().amax(-1) < 2e-4) & ((a[1] - b[1]).abs() <= 1e-3 * b[1].abs() + 1e-4)
+    assert close.float().mean() >= 0.97
