@@ -378,6 +378,16 @@ static inline size_t seed_ik_smem(const SeedIkArgs& a, int nth) {
   return seed_ik_slots_offset(a) + sizeof(float) * (size_t)a.m.n_joints * 7 * nth;
 }
 
+// What the block stages when there is room: the world up to 48 KB and, with
+// `grid`, the obstacle grid over 32 or more of its spheres.
+static inline void seed_ik_want(SeedIkArgs& a, bool grid) {
+  a.stage_world = a.w.smem_floats() * sizeof(float) <= 48 * 1024;
+  const bool want_grid = grid && a.enable_collision && a.stage_world && a.w.Ms >= 32 && a.w.Ms <= 65535;
+  // the LM kernels' default resolution (lm_grid_option) and list capacity
+  a.grid_n = want_grid ? lm_grid_option(0, a.w.Ms) : 0;
+  a.grid_entries = want_grid ? obstacle_grid_capacity(a.grid_n, a.w.Ms) : 0;
+}
+
 // Host side: extents and capacity checks and the shared-memory size (the
 // world is staged when it fits; with `grid`, a staged world of 32 or more
 // spheres gets the obstacle grid), argument packing, null-buffer checks.
@@ -388,11 +398,7 @@ static inline int seed_ik_common(SeedIkArgs& a, int n_act, int n_joints, int n_e
   PK_CHECK_CAP(n_act <= 16, "at most 16 actuated joints (got %d)", n_act);
   PK_CHECK_CAP(n_ee >= 1 && n_ee <= PK_MAX_EE, "n_ee=%d must be in [1, %d]", n_ee, PK_MAX_EE);
   PK_CHECK_ARG(a.iters >= 0, "negative iteration count");
-  a.stage_world = a.w.smem_floats() * sizeof(float) <= 48 * 1024;
-  const bool want_grid = grid && a.enable_collision && a.stage_world && a.w.Ms >= 32 && a.w.Ms <= 65535;
-  // the LM kernels' default resolution (lm_grid_option) and list capacity
-  a.grid_n = want_grid ? lm_grid_option(0, a.w.Ms) : 0;
-  a.grid_entries = want_grid ? obstacle_grid_capacity(a.grid_n, a.w.Ms) : 0;
+  seed_ik_want(a, grid);
   size_t smem = seed_ik_smem(a, nth);
   if (smem > 200 * 1024 && a.grid_entries) {
     a.grid_entries = 0;

@@ -21,8 +21,9 @@
 //
 // B200 mapping: 32 seeds of one problem per block of 128 threads, 4 lanes
 // per seed.  The lanes of a seed hold the same state and compute the same
-// step; they split the collision penalty over the obstacles (robot spheres
-// grouped by joint, with exact bounding-sphere culling at the margin).  Each
+// step; they share out the FK of the line-search trials and split the
+// collision penalty of each over the obstacles (robot spheres grouped by
+// joint, with exact bounding-sphere culling at the margin).  Each
 // solve of the step is FP32 with one conditional FP64 refinement step
 // (damped_step_f32: the 6 n_ee x 6 n_ee dual system for one or two EEs, the
 // normal equations for more).
@@ -33,6 +34,20 @@ namespace pk {
 
 constexpr int kSqpThreads = 128;
 constexpr int kSqpTps = 4;
+
+constexpr int kSqpSets = 6;  // pose sets per seed
+
+// Weighted squared pose error.
+template <int MAXEE>
+__device__ __forceinline__ float sqp_weighted(const SeedIkArgs& a, const float (&r)[6 * MAXEE]) {
+  float w = 0.f;
+#pragma unroll
+  for (int k = 0; k < 6 * MAXEE; ++k) {
+    const float rw = r[k] * (k % 6 < 3 ? a.pos_weight : a.ori_weight);
+    w += rw * rw;
+  }
+  return w;
+}
 
 // Box-constrained step of the current point (see the file comment).
 template <int MAXA, int MAXEE>
@@ -131,97 +146,108 @@ __global__ void __launch_bounds__(kSqpThreads) sqp_kernel(SeedIkArgs a) {
   const int s = blockIdx.x * G + grp;
   if (s >= a.S) return;  // the whole seed group
   const size_t gs = (size_t)p * a.S + s;
-  const PoseSlots ps{slots + tid, (int)blockDim.x};
   auto alpha_at = [](int i) { return i == 0 ? 1.f : i == 1 ? 0.5f : i == 2 ? 0.25f : i == 3 ? 0.1f : 0.025f; };
   float cfg[MAXA], best_cfg[MAXA];
 #pragma unroll
   for (int c = 0; c < MAXA; ++c) cfg[c] = best_cfg[c] = c < n ? a.seeds[gs * n + c] : 0.f;
-  // Evaluations ev = -1 (the seed), then per iteration 0 (the current point:
-  // step) and 1..5 (the line-search trials) through one call site each of FK,
-  // residual and penalty: with a site per use the loop outgrew the instruction
-  // cache and waited for instructions more than for anything else.  The
-  // penalty at the current point is the accepted trial's, carried over; a
-  // trial whose pose error alone is not below the best so far cannot win (the
-  // penalty is >= 0 for a weight >= 0), so its penalty is not evaluated.
-  // 256 problems x 32 seeds, 8 iterations: 1131 -> 883 us, the same bits.
-  float r[6 * MAXEE], pee[3 * MAXEE], delta[MAXA];
+  // The seed, then per iteration the 5 line-search trials: lane gl runs the FK
+  // and residual of trials gl and gl + TPS, each into a pose set of its own;
+  // the lanes then split the penalty of one trial after the other.  A seed has
+  // kSqpSets pose sets, five for the trials and one (`cur`) for the current
+  // point, which an accepted trial's set becomes, so the current point needs no
+  // FK; its penalty is the accepted trial's, carried over.  A trial whose pose
+  // error alone is not below the best so far cannot win (the penalty is >= 0
+  // for a weight >= 0), so its penalty is not evaluated.  One call site each of
+  // FK and penalty: with a site per use the loop outgrew the instruction cache.
+  // 256 problems x 32 seeds, 8 iterations: 1131 us with every lane running
+  // every trial's FK and the sites apart, 883 with one site, 762 so, the same bits.
+  float delta[MAXA];
 #pragma unroll
   for (int c = 0; c < MAXA; ++c) delta[c] = 0.f;
-  float lam = a.lambda_init, pen_cur = 0.f, best_err = 0.f, curr = 0.f, best_a_err = 1e30f, best_a_pen = 0.f;
-  int best_ai = 0, it = 0, ev = -1;
+  float lam = a.lambda_init, pen_cur = 0.f, best_err = 0.f, curr = 0.f;
+  int it = 0, cur = 0;
+  bool init = true;
   for (;;) {
-    float q[MAXA];
-    const float alpha = alpha_at(ev - 1);
+    const int nt = init ? 1 : 5;
+    auto set_of = [&](int k) {  // pose set of trial k (of the seed: the current point's)
+      const int i = init ? cur : cur + 1 + k;
+      return PoseSlots{slots + grp * kSqpSets + (i >= kSqpSets ? i - kSqpSets : i), G * kSqpSets};
+    };
+    float ws0 = 0.f, ws1 = 0.f;
+#pragma unroll 1
+    for (int rd = 0; rd * TPS < nt; ++rd) {
+      const int k = rd * TPS + gl;
+      if (k >= nt) continue;
+      float q[MAXA];
+      const float alpha = alpha_at(k);
 #pragma unroll
-    for (int c = 0; c < MAXA; ++c) q[c] = ev <= 0 ? cfg[c] : clampf(cfg[c] + alpha * delta[c], sh.lo[c], sh.hi[c]);
-    fk_thread(sh.jt, [&](int i) { return reg_at(q, i); }, ps);
-    seed_ik_residual<MAXEE>(sh, ps, a.n_ee, 0, r, pee);
-    float wsq = 0.f;
-#pragma unroll
-    for (int k = 0; k < 6 * MAXEE; ++k) {
-      const float rw = r[k] * (k % 6 < 3 ? a.pos_weight : a.ori_weight);
-      wsq += rw * rw;
+      for (int c = 0; c < MAXA; ++c) q[c] = init ? cfg[c] : clampf(cfg[c] + alpha * delta[c], sh.lo[c], sh.hi[c]);
+      const PoseSlots ps = set_of(k);
+      fk_thread(sh.jt, [&](int i) { return reg_at(q, i); }, ps);
+      float r[6 * MAXEE], pee[3 * MAXEE];
+      seed_ik_residual<MAXEE>(sh, ps, a.n_ee, 0, r, pee);
+      const float w = sqp_weighted<MAXEE>(a, r);
+      if (rd == 0) ws0 = w;
+      else ws1 = w;
     }
-    if (ev == 0) {
-      bool conv = true;
-#pragma unroll
-      for (int e = 0; e < MAXEE; ++e) {
-        if (e >= a.n_ee) continue;
-        const float pn = sqrtf(r[6 * e] * r[6 * e] + r[6 * e + 1] * r[6 * e + 1] + r[6 * e + 2] * r[6 * e + 2]);
-        const float on =
-            sqrtf(r[6 * e + 3] * r[6 * e + 3] + r[6 * e + 4] * r[6 * e + 4] + r[6 * e + 5] * r[6 * e + 5]);
-        if (pn >= a.eps_pos || on >= a.eps_ori) conv = false;
-      }
-      if (conv) break;
-      curr = wsq + pen_cur;
-      sqp_direction<MAXA, MAXEE>(a, sh, ps, r, pee, cfg, lam, delta);
-      best_a_err = 1e30f;
-      best_a_pen = pen_cur;
-      best_ai = 0;
-      ev = 1;
-      continue;
-    }
-    const bool need = ev < 0 || wsq < best_a_err || !(a.collision_weight >= 0.f);  // the same on the seed's lanes
-    if (need) {
-      const float pen = seed_ik_penalty<TPS>(a, ps, R, ob, gl, gmask);
+    __syncwarp(gmask);  // the lanes' pose sets are read by the whole group
+    float best_a_err = 1e30f, best_a_pen = pen_cur;
+    int best_ai = 0;
+#pragma unroll 1
+    for (int k = 0; k < nt; ++k) {
+      const float wsq = __shfl_sync(gmask, k < TPS ? ws0 : ws1, k % TPS, TPS);
+      if (!init && !(wsq < best_a_err) && a.collision_weight >= 0.f) continue;  // the same on the seed's lanes
+      const float pen = seed_ik_penalty<TPS>(a, set_of(k), R, ob, gl, gmask);
       const float et = wsq + pen;
-      if (ev < 0) {
+      if (init) {
         pen_cur = pen;
         best_err = et;
       } else if (et < best_a_err) {
         best_a_err = et;
         best_a_pen = pen;
-        best_ai = ev - 1;
+        best_ai = k;
       }
     }
-    if (ev < 0) {
-      if (a.iters <= 0) break;
-      ev = 0;
-      continue;
-    }
-    if (ev < 5) {
-      ++ev;
-      continue;
-    }
-    float trial[MAXA];
-    const float best_alpha = alpha_at(best_ai);
+    if (!init) {
+      float trial[MAXA];
+      const float best_alpha = alpha_at(best_ai);
 #pragma unroll
-    for (int c = 0; c < MAXA; ++c) trial[c] = clampf(cfg[c] + best_alpha * delta[c], sh.lo[c], sh.hi[c]);
-    if (best_a_err < curr * (1.f - 1e-4f)) {
+      for (int c = 0; c < MAXA; ++c) trial[c] = clampf(cfg[c] + best_alpha * delta[c], sh.lo[c], sh.hi[c]);
+      if (best_a_err < curr * (1.f - 1e-4f)) {
 #pragma unroll
-      for (int c = 0; c < MAXA; ++c) cfg[c] = trial[c];
-      pen_cur = best_a_pen;
-      lam = fmaxf(lam * 0.5f, 1e-10f);
-    } else {
-      lam = fminf(lam * 3.f, 1e6f);
-    }
-    if (best_a_err < best_err) {
-      best_err = best_a_err;
+        for (int c = 0; c < MAXA; ++c) cfg[c] = trial[c];
+        pen_cur = best_a_pen;
+        cur = cur + 1 + best_ai;
+        if (cur >= kSqpSets) cur -= kSqpSets;
+        lam = fmaxf(lam * 0.5f, 1e-10f);
+      } else {
+        lam = fminf(lam * 3.f, 1e6f);
+      }
+      if (best_a_err < best_err) {
+        best_err = best_a_err;
 #pragma unroll
-      for (int c = 0; c < MAXA; ++c) best_cfg[c] = trial[c];
+        for (int c = 0; c < MAXA; ++c) best_cfg[c] = trial[c];
+      }
+      ++it;
     }
-    if (++it >= a.iters) break;
-    ev = 0;
+    if (it >= a.iters) break;
+    init = false;
+    // the current point: convergence, step
+    const PoseSlots ps{slots + grp * kSqpSets + cur, G * kSqpSets};
+    float r[6 * MAXEE], pee[3 * MAXEE];
+    seed_ik_residual<MAXEE>(sh, ps, a.n_ee, 0, r, pee);
+    bool conv = true;
+#pragma unroll
+    for (int e = 0; e < MAXEE; ++e) {
+      if (e >= a.n_ee) continue;
+      const float pn = sqrtf(r[6 * e] * r[6 * e] + r[6 * e + 1] * r[6 * e + 1] + r[6 * e + 2] * r[6 * e + 2]);
+      const float on = sqrtf(r[6 * e + 3] * r[6 * e + 3] + r[6 * e + 4] * r[6 * e + 4] + r[6 * e + 5] * r[6 * e + 5]);
+      if (pn >= a.eps_pos || on >= a.eps_ori) conv = false;
+    }
+    if (conv) break;
+    curr = sqp_weighted<MAXEE>(a, r) + pen_cur;
+    sqp_direction<MAXA, MAXEE>(a, sh, ps, r, pee, cfg, lam, delta);
+    __syncwarp(gmask);  // every lane has read the set that a rejected trial may reuse
   }
   if (gl == 0) {
     for (int c = 0; c < n; ++c) a.out[gs * n + c] = reg_at(best_cfg, c);
@@ -236,12 +262,12 @@ using namespace pk;
 namespace {
 
 template <int MAXA, int MAXEE>
-int launch_sqp(const SeedIkArgs& a, size_t smem, cudaStream_t st) {
+int launch_sqp(const SeedIkArgs& a, int threads, size_t smem, cudaStream_t st) {
   auto k = sqp_kernel<MAXA, MAXEE, kSqpTps>;
   if (int s = set_smem_limit((const void*)k, smem)) return s;
-  constexpr int G = kSqpThreads / kSqpTps;
+  const int G = threads / kSqpTps;
   const dim3 grid((unsigned)((a.S + G - 1) / G), (unsigned)a.P);
-  k<<<grid, kSqpThreads, smem, st>>>(a);
+  k<<<grid, threads, smem, st>>>(a);
   return cuda_status(cudaGetLastError(), "sqp_kernel launch");
 }
 
@@ -276,12 +302,20 @@ extern "C" int pk_sqp_ik_cuda(void* stream, const float* seeds, const float* twi
   a.enable_collision = enable_collision ? 1 : 0;
   a.collision_weight = collision_weight;
   a.collision_margin = collision_margin;
+  // fewer seeds per block where the pose sets of 32 (of a robot of many joints)
+  // leave no room for the world and its grid
+  int threads = kSqpThreads;
+  {
+    SeedIkArgs w = a;
+    seed_ik_want(w, true);
+    while (threads > 32 && n_joints > 0 && seed_ik_smem(w, threads / kSqpTps * kSqpSets) > 200 * 1024) threads >>= 1;
+  }
   size_t smem = 0;
-  if (int s = seed_ik_common(a, n_act, n_joints, n_ee, kSqpThreads, &smem, true)) return s;
+  if (int s = seed_ik_common(a, n_act, n_joints, n_ee, threads / kSqpTps * kSqpSets, &smem, true)) return s;
   if (n_problems == 0 || n_seeds == 0) return PK_OK;
   if (int s = seed_ik_check_buffers(a)) return s;
   cudaStream_t st = (cudaStream_t)stream;
-  if (n_act <= 8 && n_ee == 1) return launch_sqp<8, 1>(a, smem, st);
-  if (n_ee <= 2) return launch_sqp<16, 2>(a, smem, st);
-  return launch_sqp<16, 4>(a, smem, st);
+  if (n_act <= 8 && n_ee == 1) return launch_sqp<8, 1>(a, threads, smem, st);
+  if (n_ee <= 2) return launch_sqp<16, 2>(a, threads, smem, st);
+  return launch_sqp<16, 4>(a, threads, smem, st);
 }
