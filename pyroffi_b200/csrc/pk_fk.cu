@@ -25,7 +25,7 @@ namespace pk {
 // whole robot's poses per thread, 104 KB per block for 29 joints, left 6).  A
 // parent of an earlier chunk is read back from the output rows, which this
 // warp has written.  100,003 configurations of the 29-joint humanoid:
-// 178 -> 76 us (0.52 -> 1.2 TB/s).
+// 178 -> 76 us (0.52 -> 1.2 TB/s), 71 with the joint values loaded a joint ahead.
 constexpr int kFkChunk = 8;
 constexpr int kFkTile = kFkChunk * 7;  // floats per configuration and chunk
 
@@ -46,12 +46,18 @@ __global__ void __launch_bounds__(128, 6) fk_kernel(ModelArgs m, const float* __
   float* row = out + (b0 + (live ? lane : 0)) * nj7;
   const PoseSlots ps{tile + lane, 33};
   Pose prev = pose_identity();
+  // the joint values one joint ahead: their loads are the only long waits
+  auto value = [&](int i) {
+    const int src = i < n ? jt.src[i] : -1;
+    return src < 0 ? 0.f : __ldg(c + src);
+  };
+  float q_next = value(0);
   for (int i0 = 0; i0 < n; i0 += kFkChunk) {
     const int cn = min(kFkChunk, n - i0);
 #pragma unroll 1
     for (int i = i0; i < i0 + cn; ++i) {
-      const int src = jt.src[i];
-      const float q = ((src < 0) ? 0.f : __ldg(c + src)) * jt.mul[i] + jt.off[i];
+      const float q = q_next * jt.mul[i] + jt.off[i];
+      q_next = value(i + 1);
       const Pose Tpc = joint_local(jt, i, q);
       const int p = jt.psorted[i];
       Pose Tw;
@@ -78,11 +84,13 @@ __global__ void __launch_bounds__(128, 6) fk_kernel(ModelArgs m, const float* __
       const int r0 = e / kFkTile, col = e - r0 * kFkTile;
       if (col >= cn * 7) continue;
       const int jj = col / 7;
-      const int at = jt.orig[i0 + jj] * 7 + (col - jj * 7);
+      const float* from = tile + col * 33 + r0;
+      float* to = dst + r0 * nj7 + jt.orig[i0 + jj] * 7 + (col - jj * 7);
+      if (rows == 32) {
 #pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        const int r = r0 + 4 * g;
-        if (r < rows) dst[(long long)r * nj7 + at] = tile[col * 33 + r];
+        for (int g = 0; g < 8; ++g) to[4 * g * nj7] = from[4 * g];
+      } else {
+        for (int r = r0; r < rows; r += 4, from += 4, to += 4 * nj7) *to = *from;
       }
     }
     __syncwarp();
