@@ -93,7 +93,7 @@ def odd_robot(n_joints):
     from pyroffi_b200.robot import RobotModel
     rng = np.random.default_rng(n_joints)
     n = n_joints
-    parent = np.array([2, 0, -1, 2, 3, 4, 5, 6, 3][:n])
+    parent = np.array([2, 0, -1, 2, 3, 4, 5, 6, 3][:n] if n > 2 else [-1] * n)
     kinds = ["rev", "rev", "pris", "fixed", "rev", "rev", "rev", "rev", "rev"][:n]
     twists, ptf = np.zeros((n, 6)), np.zeros((n, 7))
     act, mimic, mul, off = -np.ones(n, int), -np.ones(n, int), np.ones(n), np.zeros(n)
