@@ -288,6 +288,8 @@ __device__ __forceinline__ void narrow_world(const PenaltyCtx& c, const Pose& T,
   o.x += jb.x; o.y += jb.y; o.z += jb.z;
   const float2 nx = make_float2(-o.x, -o.x), ny = make_float2(-o.y, -o.y), nz = make_float2(-o.z, -o.z);
   const float2 ow = make_float2(O.w, O.w);
+  float2 sum = make_float2(0.f, 0.f);
+#pragma unroll 2
   for (int p = p0; p < p1; ++p) {
     const float4 s0 = c.rsp[2 * p], s1 = c.rsp[2 * p + 1];
     const float2 dx = __fadd2_rn(make_float2(s0.x, s0.y), nx);
@@ -296,10 +298,9 @@ __device__ __forceinline__ void narrow_world(const PenaltyCtx& c, const Pose& T,
     float2 d2 = __fmul2_rn(dx, dx);
     d2 = __ffma2_rn(dy, dy, d2);
     d2 = __ffma2_rn(dz, dz, d2);
-    const float2 rr = __fadd2_rn(make_float2(s1.z, s1.w), ow);
-    hinge_sq(d2.x, rr.x, pen);
-    hinge_sq(d2.y, rr.y, pen);
+    hinge_add2(d2, __fadd2_rn(make_float2(s1.z, s1.w), ow), sum);
   }
+  pen += sum.x + sum.y;
 }
 
 // Hinge terms of the pairs of self-pair group gi of one seed (poses in ps),
@@ -330,6 +331,7 @@ __device__ __forceinline__ void group_pairs(const PenaltyCtx& c, const PoseSlots
   u.z += cx.z - (m20.x * cy.x + m21.x * cy.y + m22.x * cy.z);
   const float2 ux = dup(u.x), uy = dup(u.y), uz = dup(u.z);
   // two pairs per packed FP32x2 operation: e = M c_b + u - c_a
+  float2 sum = make_float2(0.f, 0.f);
   const int q1 = c.pgstart[gi + 1];
   for (int q = c.pgstart[gi]; q < q1; q += 2) {
     const float4 r0 = c.prec[2 * q], r1 = c.prec[2 * q + 1], r2 = c.prec[2 * q + 2], r3 = c.prec[2 * q + 3];
@@ -340,9 +342,9 @@ __device__ __forceinline__ void group_pairs(const PenaltyCtx& c, const PoseSlots
     float2 d2 = __fmul2_rn(ex, ex);
     d2 = __ffma2_rn(ey, ey, d2);
     d2 = __ffma2_rn(ez, ez, d2);
-    if (d2.x < r3.z) { const float e = sqrtf(d2.x) - r1.z; pen += e * e; }
-    if (d2.y < r3.w) { const float e = sqrtf(d2.y) - r1.w; pen += e * e; }
+    hinge_add2(d2, make_float2(r1.z, r1.w), sum);
   }
+  pen += sum.x + sum.y;
 }
 
 // Self pairs of one seed, split over its TPS lanes (TPS > 1): the

@@ -505,10 +505,11 @@ __device__ __noinline__ float w_penalty(const WideLaunch& P, const WideShared& s
       if (dx * dx + dy * dy + dz * dz < rr * fabsf(rr)) {
         // the obstacle in the joint's frame, against the joint's spheres there
         const float3 o = pose_apply_inv(w_load(W.T, sh.js_joint[j]), make_float3(O.x, O.y, O.z));
+        const float2 no = make_float2(-o.x, -o.y), ow = make_float2(-o.z, O.w);
+#pragma unroll 4
         for (int k = sh.jstart[j]; k < sh.jstart[j + 1]; ++k) {
-          const float4 q = rs4[k];
-          const float ex = q.x - o.x, ey = q.y - o.y, ez = q.z - o.z;
-          w_hinge(ex * ex + ey * ey + ez * ez, q.w + O.w, pen);
+          const float2 g = sphere_gap(rs4[k], no, ow);
+          hinge_add(g.x, g.y, pen);
         }
       }
     }

@@ -304,8 +304,7 @@ __device__ __forceinline__ void seed_ik_jacobian(const SeedIkShared& sh, const P
 // exactly 0 for every sphere of the group and is skipped; with the grid, the
 // world spheres tested are those listed in the cell of the group's bounding
 // centre.  A world sphere that passes is moved into the joint's frame once
-// and tested against the group's spheres there on squared distances (a
-// square root only for a hit); the other kinds are tested in the world frame.
+// and tested against the group's spheres there; the other kinds are tested in the world frame.
 template <int TPS>
 __device__ __forceinline__ float seed_ik_penalty(const SeedIkArgs& a, const PoseSlots& ps, const RobotSpheresS& R,
                                               const ObsView& ob, int gl, unsigned gmask) {
@@ -333,15 +332,11 @@ __device__ __forceinline__ float seed_ik_penalty(const SeedIkArgs& a, const Pose
     auto narrow_sphere = [&](int m) {
       const float4 O = ob.sph[m];
       const float3 o = pose_apply_inv(Tj, make_float3(O.x, O.y, O.z));
+      const float2 no = make_float2(-o.x, -o.y), ow = make_float2(-o.z, O.w);
+#pragma unroll 4
       for (int i = R.gstart[k]; i < R.gstart[k + 1]; ++i) {
-        const float4 q = R.sph[i];
-        const float dx = q.x - o.x, dy = q.y - o.y, dz = q.z - o.z;
-        const float d2 = dx * dx + dy * dy + dz * dz;
-        const float rr = q.w + O.w + margin;
-        if (d2 < rr * fabsf(rr)) {
-          const float e = sqrtf(d2) - rr;
-          pen += e * e;
-        }
+        const float2 g = sphere_gap(R.sph[i], no, ow);
+        hinge_add(g.x, g.y + margin, pen);
       }
     };
     if (R.cell_start) {

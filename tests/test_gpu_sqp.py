@@ -117,3 +117,23 @@ def test_partial_seed_blocks_and_empty_batch():
         assert np.all(cfg[p] >= w.model.lower - 1e-6) and np.all(cfg[p] <= w.model.upper + 1e-6)
     c0, e0 = sol.run(t(w.seeds[:0]), t(w.target_T[:0]), max_iter=5, **KW)
     assert c0.shape == (0, 33, w.model.n_act) and e0.shape == (0, 33)
+
+
+@pytest.mark.parametrize("n_joints", [30, 40, 64])
+def test_smaller_blocks_for_robots_of_many_joints(n_joints):
+    """Fixed leaf joints at the root change no pose of the arm, but their pose
+    sets leave room for fewer seeds per block: the same bits as without them."""
+    from pyroffi_b200.robot import RobotModel
+    w, sol, *_ = chain(P=2, S=33, coll=True)
+    m, k = w.model, n_joints - w.model.n_joints
+    ident = np.tile(np.array([1.0, 0, 0, 0, 0, 0, 0]), (k, 1))
+    pad = lambda x, v: np.concatenate([np.asarray(x), np.full(k, v, np.asarray(x).dtype)])
+    big = RobotModel(twists=np.concatenate([m.twists, np.zeros((k, 6))]),
+                     parent_tf=np.concatenate([m.parent_tf, ident]), parent_idx=pad(m.parent_idx, -1),
+                     act_idx=pad(m.act_idx, -1), mimic_mul=pad(m.mimic_mul, 1.0), mimic_off=pad(m.mimic_off, 0.0),
+                     mimic_act_idx=pad(m.mimic_act_idx, -1), parent_joint_indices=m.parent_joint_indices,
+                     lower=m.lower, upper=m.upper)
+    padded = SqpSolver(big, w.target_link, spheres=w.spheres, world=w.world, enable_collision=True, device=DEV)
+    a = sol.run(t(w.seeds), t(w.target_T), max_iter=8, **KW)
+    b = padded.run(t(w.seeds), t(w.target_T), max_iter=8, **KW)
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
