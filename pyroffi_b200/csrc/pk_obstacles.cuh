@@ -427,17 +427,6 @@ __device__ __forceinline__ void near_of_kind(const ObsView& ob, Index index, int
   }
 }
 
-// The same for all obstacles of the kinds other than spheres: one pass per
-// kind, so neither the test nor f needs to dispatch.
-template <class F>
-__device__ __forceinline__ void for_each_near_other(const ObsView& ob, float3 B, float R, float margin, int lane,
-                                                    int stride, F&& f) {
-  const int b1 = ob.Ms, b2 = b1 + ob.Mc, b3 = b2 + ob.Mb;
-  near_of_kind<1>(ob, [=](int i) { return b1 + i; }, ob.Mc, B, R, margin, lane, stride, f);
-  near_of_kind<2>(ob, [=](int i) { return b2 + i; }, ob.Mb, B, R, margin, lane, stride, f);
-  near_of_kind<3>(ob, [=](int i) { return b3 + i; }, ob.Mh, B, R, margin, lane, stride, f);
-}
-
 __device__ __forceinline__ float3 cross3(float3 a, float3 b) {
   return make_float3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }

@@ -25,6 +25,7 @@
 #include <float.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "pk_obstacles.cuh"
 
@@ -51,10 +52,25 @@ struct TrajArgs {
   long long active_period;
 };
 
+// Bounding sphere of a capsule or a box (the list's slack covers its rounding).
+__device__ __forceinline__ float4 capsule_ball(const float* c) {
+  const float hx = 0.5f * (c[3] - c[0]), hy = 0.5f * (c[4] - c[1]), hz = 0.5f * (c[5] - c[2]);
+  return make_float4(c[0] + hx, c[1] + hy, c[2] + hz, c[6] + sqrtf(hx * hx + hy * hy + hz * hz));
+}
+__device__ __forceinline__ float4 box_ball(const float* b) {
+  return make_float4(b[0], b[1], b[2], sqrtf(b[12] * b[12] + b[13] * b[13] + b[14] * b[14]));
+}
+
+// Obstacles that a warp's candidate list has room for: all but the halfspaces.
+__host__ __device__ __forceinline__ int listed(const WorldArgs& w) { return w.Ms + w.Mc + w.Mb; }
+
 // Lanes per waypoint: the world (link, obstacle) pairs and the self pairs of
 // one waypoint are split over a group of TG lanes (TG = 2 or 4); its FK,
 // force totals and joint gradient live once per waypoint in shared memory.
-template <int MAXS, int TG>
+// GRAD: the gradient is wanted; a cost needs neither the sphere that attains a
+// minimum nor the forces, and its launch is the more frequent one (a line
+// search costs five trajectories per gradient).
+template <int MAXS, int TG, bool GRAD>
 __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if (a.active && !a.active[blockIdx.x % a.active_period]) return;  // block-uniform: nothing is written
@@ -74,8 +90,8 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
   float* slots = reinterpret_cast<float*>(p); p += sizeof(float) * nj * 7 * ng;   // per waypoint group
   float* lt = reinterpret_cast<float*>(p); p += sizeof(float) * N * 6 * ng;       // link force / moment totals
   float* gq = reinterpret_cast<float*>(p); p += sizeof(float) * nj * ng;          // gradient per joint
-  unsigned short* cand = reinterpret_cast<unsigned short*>(p) + (size_t)(tid >> 5) * a.w.Ms;  // this warp's candidates
-  if (a.list) p += sizeof(unsigned short) * (size_t)a.w.Ms * (nth >> 5);
+  unsigned short* cand = reinterpret_cast<unsigned short*>(p) + (size_t)(tid >> 5) * listed(a.w);  // this warp's candidates
+  if (a.list) p += sizeof(unsigned short) * (size_t)listed(a.w) * (nth >> 5);
   p = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15));
 
   load_joint_table(jt, a.m);
@@ -114,7 +130,7 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
   }
   __syncthreads();
 
-  const bool want_grad = a.grad != nullptr;
+  constexpr bool want_grad = GRAD;
   const float margin = a.margin;
   for (int t0 = 0; t0 < T; t0 += ng) {
     const int t = t0 + grp;
@@ -165,14 +181,18 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
             d.x = obstacle_dist<K>(ob, m, make_float3(ls.x[q].x, ls.y[q].x, ls.z[q].x), ls.r[q].x);
             d.y = obstacle_dist<K>(ob, m, make_float3(ls.x[q].y, ls.y[q].y, ls.z[q].y), ls.r[q].y);
           }
-          if (d.x < dmin) { dmin = d.x; arg = 2 * q; }
-          if (d.y < dmin) { dmin = d.y; arg = 2 * q + 1; }
+          if constexpr (GRAD) {
+            if (d.x < dmin) { dmin = d.x; arg = 2 * q; }
+            if (d.y < dmin) { dmin = d.y; arg = 2 * q + 1; }
+          } else {
+            dmin = fminf(dmin, fminf(d.x, d.y));
+          }
         }
         // padded spheres read about 1e30: a link of padding only has no hit
         if (!(dmin < margin)) return;
         const float v = margin - dmin;
         cw += v * v;
-        if (want_grad) {
+        if constexpr (GRAD) {
           float3 c = make_float3(0.f, 0.f, 0.f), g;
           float rr = 0.f;
 #pragma unroll
@@ -186,33 +206,48 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
           Mo.x += cm.x; Mo.y += cm.y; Mo.z += cm.z;
         }
       };
-      // World spheres within reach of the box around the warp's (consecutive)
-      // waypoints of this link, listed once per warp; each waypoint's lanes
-      // then test only those, where testing every sphere was most of the
-      // kernel's work: cost and gradient launches of 512 x 64 x 7 among 288
-      // obstacles 293 -> 205 us, five CHOMP iterations 4181 -> 3069 us.
+      // World spheres, capsules and boxes whose bounding spheres are within
+      // reach of the box around the warp's (consecutive) waypoints of this link,
+      // listed once per warp; each waypoint's lanes then test only those, where
+      // testing every obstacle was most of the kernel's work: cost and gradient
+      // launches of 512 x 64 x 7 among 288 obstacles 293 -> 205 us with the
+      // spheres listed, 205 -> 180 with the capsules and boxes listed too and the
+      // cost apart from the gradient (five CHOMP iterations 3069 -> 2554)
       const float3 bl3 = make_float3(warp_min_of(wm, B.x), warp_min_of(wm, B.y), warp_min_of(wm, B.z));
       const float3 bh3 = make_float3(warp_max_of(wm, B.x), warp_max_of(wm, B.y), warp_max_of(wm, B.z));
       const int lane = tid & 31, step = __popc(wm);
-      int n_cand = a.list ? 0 : ob.Ms;
-      for (int k0 = 0; k0 < (a.list ? ob.Ms : 0); k0 += step) {
-        const int k = k0 + lane;
-        bool in = false;
-        if (k < ob.Ms) {
-          const float4 o = ob.sph[k];
-          const float dx = fmaxf(fmaxf(bl3.x - o.x, o.x - bh3.x), 0.f), dy = fmaxf(fmaxf(bl3.y - o.y, o.y - bh3.y), 0.f),
-                      dz = fmaxf(fmaxf(bl3.z - o.z, o.z - bh3.z), 0.f);
-          const float r0 = bl.w + margin + o.w, rr = r0 + 1e-4f + 1e-5f * fabsf(r0);  // rounding slack
-          // not "<": a NaN pose or obstacle stays a candidate, as without the list
-          in = !(dx * dx + dy * dy + dz * dz >= rr * fabsf(rr));
+      int n_cand = 0;
+      // lists obstacles base, base + 1, ... (ball(k): the bounding sphere of the k-th); returns their number
+      auto list_kind = [&](int base, int count, auto ball) {
+        if (!a.list) return count;
+        const int first = n_cand;
+        for (int k0 = 0; k0 < count; k0 += step) {
+          const int k = k0 + lane;
+          bool in = false;
+          if (k < count) {
+            const float4 o = ball(k);
+            const float dx = fmaxf(fmaxf(bl3.x - o.x, o.x - bh3.x), 0.f), dy = fmaxf(fmaxf(bl3.y - o.y, o.y - bh3.y), 0.f),
+                        dz = fmaxf(fmaxf(bl3.z - o.z, o.z - bh3.z), 0.f);
+            const float r0 = bl.w + margin + o.w, rr = r0 + 1e-4f + 1e-5f * fabsf(r0);  // rounding slack
+            // not "<": a NaN pose or obstacle stays a candidate, as without the list
+            in = !(dx * dx + dy * dy + dz * dz >= rr * fabsf(rr));
+          }
+          const unsigned m = __ballot_sync(wm, in);
+          if (in) cand[n_cand + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(base + k);
+          n_cand += __popc(m);
         }
-        const unsigned m = __ballot_sync(wm, in);
-        if (in) cand[n_cand + __popc(m & ((1u << lane) - 1u))] = (unsigned short)k;
-        n_cand += __popc(m);
-      }
+        return n_cand - first;
+      };
+      const int b1 = ob.Ms, b2 = b1 + ob.Mc, b3 = b2 + ob.Mb;
+      const int n0 = list_kind(0, ob.Ms, [&](int k) { return ob.sph[k]; });
+      const int n1 = list_kind(b1, ob.Mc, [&](int k) { return capsule_ball(ob.cap + 7 * k); });
+      const int n2 = list_kind(b2, ob.Mb, [&](int k) { return box_ball(ob.box + 15 * k); });
       __syncwarp(wm);
-      near_of_kind<0>(ob, [&](int i) { return a.list ? (int)cand[i] : i; }, n_cand, B, bl.w, margin, gl, TG, narrow);
-      for_each_near_other(ob, B, bl.w, margin, gl, TG, narrow);
+      near_of_kind<0>(ob, [&](int i) { return a.list ? (int)cand[i] : i; }, n0, B, bl.w, margin, gl, TG, narrow);
+      near_of_kind<1>(ob, [&](int i) { return a.list ? (int)cand[n0 + i] : b1 + i; }, n1, B, bl.w, margin, gl, TG, narrow);
+      near_of_kind<2>(ob, [&](int i) { return a.list ? (int)cand[n0 + n1 + i] : b2 + i; }, n2, B, bl.w, margin, gl, TG,
+                      narrow);
+      near_of_kind<3>(ob, [=](int i) { return b3 + i; }, ob.Mh, B, bl.w, margin, gl, TG, narrow);
       __syncwarp(wm);  // the next link's list goes in the same place
       if (want_grad) {
 #pragma unroll
@@ -392,7 +427,7 @@ static size_t traj_smem(const TrajArgs& a, int nth, int TG) {
              2 * sizeof(float) * ((a.T * a.m.n_act + 3) & ~3) + sizeof(float) * ((nth + 3) & ~3) +
              sizeof(float) * ((a.T + 3) & ~3) +
              sizeof(float) * (size_t)(nth / TG) * (a.m.n_joints * 7 + a.N * 6 + a.m.n_joints) +
-             (a.list ? sizeof(unsigned short) * (size_t)a.w.Ms * (nth / 32) : 0);
+             (a.list ? sizeof(unsigned short) * (size_t)listed(a.w) * (nth / 32) : 0);
   s = (s + 15) & ~size_t(15);
   return s + sizeof(float) * a.w.smem_floats();
 }
@@ -452,7 +487,7 @@ extern "C" int pk_traj_cost_grad(void* stream, const pk_traj_options* opt, const
   // the candidate lists where they cost no resident block
   a.list = 0;
   size_t smem = traj_smem(a, nth, TG);
-  if (Ms > 0) {
+  if (listed(a.w) > 0) {
     a.list = 1;
     const size_t with = traj_smem(a, nth, TG);
     auto per_sm = [&](size_t b) { return std::min<size_t>(512 / nth, (228 * 1024) / (b + 1024)); };  // 128 registers
@@ -461,9 +496,13 @@ extern "C" int pk_traj_cost_grad(void* stream, const pk_traj_options* opt, const
   }
   PK_CHECK_CAP(smem <= 200 * 1024, "trajectory working set (%zu B of shared memory) too large", smem);
   PK_CHECK_CAP(B < (1LL << 31), "batch too large");
-  auto kern = (S <= 8)    ? (TG == 4 ? traj_cost_kernel<8, 4> : traj_cost_kernel<8, 2>)
-              : (S <= 16) ? (TG == 4 ? traj_cost_kernel<16, 4> : traj_cost_kernel<16, 2>)
-                          : (TG == 4 ? traj_cost_kernel<32, 4> : traj_cost_kernel<32, 2>);
+  auto pick = [&](auto gradient) {
+    constexpr bool G = decltype(gradient)::value;
+    return (S <= 8)    ? (TG == 4 ? traj_cost_kernel<8, 4, G> : traj_cost_kernel<8, 2, G>)
+           : (S <= 16) ? (TG == 4 ? traj_cost_kernel<16, 4, G> : traj_cost_kernel<16, 2, G>)
+                       : (TG == 4 ? traj_cost_kernel<32, 4, G> : traj_cost_kernel<32, 2, G>);
+  };
+  auto kern = grad ? pick(std::true_type()) : pick(std::false_type());
   if (int s = set_smem_limit((const void*)kern, smem)) return s;
   kern<<<(unsigned)B, nth, smem, (cudaStream_t)stream>>>(a);
   return cuda_status(cudaGetLastError(), "traj_cost_kernel launch");
