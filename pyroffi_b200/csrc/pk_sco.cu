@@ -132,8 +132,18 @@ __device__ __forceinline__ float group_sum(float v, unsigned gm) {
   return v;
 }
 
+// (x, y, z) to unit length by the approximate reciprocal root and one Newton
+// step (about an ulp); 0 stays 0.
+__device__ __forceinline__ float3 unit_from(float x, float y, float z) {
+  const float d2 = x * x + y * y + z * z;
+  float i = rsqrt_approx(d2 + 1e-30f);
+  i = i * fmaf(-0.5f * d2, i * i, 1.5f);
+  return make_float3(x * i, y * i, z * i);
+}
+
 // One world obstacle of a known kind in registers (1 sphere, 2 capsule, 3
-// box, 4 halfspace) and its signed distance to a sphere (c, r).
+// box, 4 halfspace), its signed distance to a sphere (c, r) and that distance's
+// gradient with respect to c.
 template <int KIND>
 struct ScoObs;
 
@@ -148,6 +158,7 @@ struct ScoObs<1> {
     const float dx = cx - x, dy = cy - y, dz = cz - z;
     return sqrt_fast(dx * dx + dy * dy + dz * dz) - (cr + r);
   }
+  __device__ __forceinline__ float3 grad(float3 c) const { return unit_from(c.x - x, c.y - y, c.z - z); }
 };
 
 template <>
@@ -167,6 +178,11 @@ struct ScoObs<2> {
     const float px = fmaf(t, vx, ax) - cx, py = fmaf(t, vy, ay) - cy, pz = fmaf(t, vz, az) - cz;
     return sqrt_fast(px * px + py * py + pz * pz) - (cr + r);
   }
+  __device__ __forceinline__ float3 grad(float3 c) const {
+    float t = ((c.x - ax) * vx + (c.y - ay) * vy + (c.z - az) * vz) * il2;
+    t = fmaxf(0.f, fminf(1.f, t));
+    return unit_from(c.x - fmaf(t, vx, ax), c.y - fmaf(t, vy, ay), c.z - fmaf(t, vz, az));
+  }
 };
 
 template <>
@@ -184,6 +200,22 @@ struct ScoObs<3> {
     const float m1 = fmaxf(q1, 0.f), m2 = fmaxf(q2, 0.f), m3 = fmaxf(q3, 0.f);
     return sqrt_fast(m1 * m1 + m2 * m2 + m3 * m3) + fminf(fmaxf(fmaxf(q1, q2), q3), 0.f) - cr;
   }
+  // towards the nearest point of the box from outside, along the nearest face's axis inside
+  __device__ __forceinline__ float3 grad(float3 c) const {
+    const float dx = c.x - p[0], dy = c.y - p[1], dz = c.z - p[2];
+    const float l1 = dx * p[3] + dy * p[4] + dz * p[5], l2 = dx * p[6] + dy * p[7] + dz * p[8],
+                l3 = dx * p[9] + dy * p[10] + dz * p[11];
+    const float q1 = fabsf(l1) - p[12], q2 = fabsf(l2) - p[13], q3 = fabsf(l3) - p[14];
+    float3 g = unit_from(fmaxf(q1, 0.f), fmaxf(q2, 0.f), fmaxf(q3, 0.f));
+    if (g.x + g.y + g.z == 0.f) {
+      if (q1 >= q2 && q1 >= q3) g.x = 1.f;
+      else if (q2 >= q3) g.y = 1.f;
+      else g.z = 1.f;
+    }
+    g.x = copysignf(g.x, l1); g.y = copysignf(g.y, l2); g.z = copysignf(g.z, l3);
+    return make_float3(g.x * p[3] + g.y * p[6] + g.z * p[9], g.x * p[4] + g.y * p[7] + g.z * p[10],
+                       g.x * p[5] + g.y * p[8] + g.z * p[11]);
+  }
 };
 
 template <>
@@ -197,6 +229,7 @@ struct ScoObs<4> {
   __device__ __forceinline__ float dist(float cx, float cy, float cz, float cr) const {
     return cx * nx + cy * ny + cz * nz - off - cr;
   }
+  __device__ __forceinline__ float3 grad(float3) const { return make_float3(nx, ny, nz); }
 };
 
 // Terms whose softmax weight is below exp(-kScoSkip) of the running maximum
@@ -212,8 +245,8 @@ constexpr float kScoSkip = 20.f;
 // the collision sum wanted, its distance at or above the margin).
 template <int KIND, int MAXS, int TG>
 __device__ __forceinline__ SoftAcc world_group(const ScoLinArgs& a, const ObsView& ob, int base, int count, int gl,
-                                               unsigned gm, const LinkSpheres<MAXS>& L, const float4* link_sph,
-                                               const Pose& Tl, float3 B, float R, bool want_soft, bool want_j,
+                                               unsigned gm, const LinkSpheres<MAXS>& L, const float4* placed,
+                                               float3 B, float R, bool want_soft, bool want_j,
                                                float inv_tau, float gref, float& csum) {
   SoftAcc acc;
   acc.init();
@@ -264,23 +297,13 @@ __device__ __forceinline__ SoftAcc world_group(const ScoLinArgs& a, const ObsVie
     if (e < fmaxf(acc.ref, gref) - kScoSkip) continue;
     float3 cc = make_float3(0.f, 0.f, 0.f), gg = cc;
     if (want_j) {
-      // the attaining sphere, placed again from the link frame (a register
-      // array cannot be indexed by `arg`, and picking it out of MAXS costs
-      // more); with the root below and the ranking pass's survivor masks, one
-      // SCO step of 512 x 64 x 7 among 305 obstacles 1661 -> 1589 us
-      const float4 ls = link_sph[arg];
-      cc = pose_apply(Tl, make_float3(ls.x, ls.y, ls.z));
-      if constexpr (KIND == 1) {
-        // (c - o) / |c - o| by the approximate reciprocal root and one Newton
-        // step (about an ulp); 0 where the centres coincide
-        gg = make_float3(cc.x - o.x, cc.y - o.y, cc.z - o.z);
-        const float d2 = gg.x * gg.x + gg.y * gg.y + gg.z * gg.z;
-        float y = rsqrt_approx(d2 + 1e-30f);
-        y = y * fmaf(-0.5f * d2, y * y, 1.5f);
-        gg.x *= y; gg.y *= y; gg.z *= y;
-      } else {
-        obstacle_dist_grad<KIND - 1>(ob, base + k, cc, ls.w, gg);
-      }
+      // the attaining sphere from the link's placed ones (a register array
+      // cannot be indexed by `arg`, and picking it out of MAXS costs more), and
+      // the gradient from the obstacle in registers: one step of
+      // 512 x 64 x 7 trajectories among 305 obstacles 1589 -> 1441 us
+      const float4 ls = placed[arg];
+      cc = make_float3(ls.x, ls.y, ls.z);
+      gg = o.grad(cc);
     }
     acc.add(e, true, want_j, gg, cc);
   }
@@ -307,6 +330,7 @@ __global__ void __launch_bounds__(128, MAXS <= 8 ? 4 : (MAXS <= 16 ? 3 : 2)) sco
   int* lps = reinterpret_cast<int*>(p); p += sizeof(int) * (N + 1);  // CSR start of each link's self pairs
   int* lpl = reinterpret_cast<int*>(p); p += sizeof(int) * 2 * P;    // entries 2 * pair + role
   p = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15));
+  float4* placed = reinterpret_cast<float4*>(p) + grp * (MAXS + 1); p += sizeof(float4) * (MAXS + 1) * ng;  // odd stride
   float* slots = reinterpret_cast<float*>(p); p += sizeof(float) * nj * 7 * ng;
   float* gjs = reinterpret_cast<float*>(p); p += sizeof(float) * nj * nth;
   p = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15));
@@ -384,32 +408,36 @@ __global__ void __launch_bounds__(128, MAXS <= 8 ? 4 : (MAXS <= 16 ? 3 : 2)) sco
     for (int l = 0; l < N; ++l) {
       if (lcnt[l] == 0) continue;
       const Pose Tl = lpj[l] < 0 ? pose_identity() : ps.load(lpj[l]);
+      // the link's spheres, placed once by the lanes of the waypoint; a padded
+      // sphere's distances read 1e30
+      for (int i = gl; i < MAXS; i += TG) {
+        const float4 w0 = i < S ? lsph[l * S + i] : make_float4(0.f, 0.f, 0.f, -1.f);
+        const float3 v0 = pose_apply(Tl, make_float3(w0.x, w0.y, w0.z));
+        placed[i] = make_float4(v0.x, v0.y, v0.z, w0.w < 0.f ? -1e30f : w0.w);
+      }
+      __syncwarp(gm);
       LinkSpheres<MAXS> ls;
 #pragma unroll
       for (int q = 0; q < MAXS / 2; ++q) {
-        const float4 w0 = (2 * q < S) ? lsph[l * S + 2 * q] : make_float4(0.f, 0.f, 0.f, -1.f);
-        const float4 w1 = (2 * q + 1 < S) ? lsph[l * S + 2 * q + 1] : make_float4(0.f, 0.f, 0.f, -1.f);
-        const float3 v0 = pose_apply(Tl, make_float3(w0.x, w0.y, w0.z));
-        const float3 v1 = pose_apply(Tl, make_float3(w1.x, w1.y, w1.z));
+        const float4 v0 = placed[2 * q], v1 = placed[2 * q + 1];
         ls.x[q] = make_float2(v0.x, v1.x); ls.y[q] = make_float2(v0.y, v1.y); ls.z[q] = make_float2(v0.z, v1.z);
-        // a padded sphere's distances read 1e30
-        ls.r[q] = make_float2(w0.w < 0.f ? -1e30f : w0.w, w1.w < 0.f ? -1e30f : w1.w);
+        ls.r[q] = make_float2(v0.w, v1.w);
       }
       const float4 bl = lbnd[l];
       const float3 Bw = pose_apply(Tl, make_float3(bl.x, bl.y, bl.z));
       // world groups: (link, obstacle) pairs, lane gl takes obstacles gl, gl + TG, ...
       SoftAcc mine, t;
       mine.init();
-      t = world_group<1, MAXS, TG>(a, ob, 0, Ms, gl, gm, ls, lsph + l * S, Tl, Bw, bl.w, want_soft,
+      t = world_group<1, MAXS, TG>(a, ob, 0, Ms, gl, gm, ls, placed, Bw, bl.w, want_soft,
                                    want_j, inv_tau, gref[1], csum);
       if (gl == 1) mine = t;
-      t = world_group<2, MAXS, TG>(a, ob, Ms, Mc, gl, gm, ls, lsph + l * S, Tl, Bw, bl.w, want_soft,
+      t = world_group<2, MAXS, TG>(a, ob, Ms, Mc, gl, gm, ls, placed, Bw, bl.w, want_soft,
                                    want_j, inv_tau, gref[2], csum);
       if (gl == 2) mine = t;
-      t = world_group<3, MAXS, TG>(a, ob, Ms + Mc, Mb, gl, gm, ls, lsph + l * S, Tl, Bw, bl.w, want_soft,
+      t = world_group<3, MAXS, TG>(a, ob, Ms + Mc, Mb, gl, gm, ls, placed, Bw, bl.w, want_soft,
                                    want_j, inv_tau, gref[3], csum);
       if (gl == 3) mine = t;
-      t = world_group<4, MAXS, TG>(a, ob, Ms + Mc + Mb, a.w.Mh, gl, gm, ls, lsph + l * S, Tl, Bw, bl.w, want_soft,
+      t = world_group<4, MAXS, TG>(a, ob, Ms + Mc + Mb, a.w.Mh, gl, gm, ls, placed, Bw, bl.w, want_soft,
                                    want_j, inv_tau, gref[4], csum);
       if (gl == 4) mine = t;
       // self group: the pairs listing link l; lane gl takes entries gl, gl + TG, ...
@@ -1202,20 +1230,26 @@ __global__ void sco_fd_jac_kernel(const float* dfd, float* dist, float* jac, lon
   }
 }
 
-static size_t lin_smem(const ScoLinArgs& a, int nth, int TG) {
+// `placed`: float4 of a waypoint's placed link spheres
+static size_t lin_smem(const ScoLinArgs& a, int nth, int TG, int placed) {
   const int ng = nth / TG, nj = a.m.n_joints;
   size_t s = sizeof(JointTable) + sizeof(float4) * a.N * (a.S + 1) + sizeof(int) * (3 * a.N + a.N + 1 + 2 * a.P);
   s = (s + 15) & ~size_t(15);
-  s += sizeof(float) * ((size_t)nj * 7 * ng + (size_t)nj * nth);
+  s += sizeof(float4) * (size_t)placed * ng + sizeof(float) * ((size_t)nj * 7 * ng + (size_t)nj * nth);
   s = (s + 15) & ~size_t(15);
   return s + sizeof(float) * a.w.smem_floats();
 }
 
 static int launch_linearize(const ScoLinArgs& a, cudaStream_t st) {
   if (a.C == 0) return PK_OK;
-  constexpr int TG = 8, nth = 128;
-  const size_t smem = lin_smem(a, nth, TG);
-  PK_CHECK_CAP(smem <= 220 * 1024, "SCO linearisation working set (%zu B of shared memory) too large", smem);
+  constexpr int TG = 8;
+  const size_t need = lin_smem(a, 128, TG, 0);
+  PK_CHECK_CAP(need <= 220 * 1024, "SCO linearisation working set (%zu B of shared memory) too large", need);
+  // fewer waypoints per block where the placed spheres of 16 do not fit
+  const int placed = (a.S <= 4 ? 4 : a.S <= 8 ? 8 : a.S <= 16 ? 16 : 32) + 1;
+  int nth = 128;
+  while (nth > 32 && lin_smem(a, nth, TG, placed) > 226 * 1024) nth >>= 1;
+  const size_t smem = lin_smem(a, nth, TG, placed);
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const long long ng = nth / TG;
