@@ -24,9 +24,9 @@
 // within (eps_pos, eps_ori) stops, and so do the other seeds of its problem
 // from the next iteration on.
 //
-// B200 mapping.  Coarse: eight lanes per seed for robots of up to 8 joints,
-// else one thread per seed; grid (seed blocks, problems), robot, limits, world
-// and robot spheres in shared memory.  Refinement: one 128-thread block per problem,
+// B200 mapping.  Coarse: one thread per seed, grid (seed blocks, problems),
+// robot, limits, world and robot spheres in shared memory, joint poses in
+// per-thread shared slots.  Refinement: one 128-thread block per problem,
 // four lanes per refinement seed (32 seeds at a time; the four lanes split
 // the collision penalty); the problem's stop flag is a block vote
 // (__syncthreads_or), so every seed of a problem stops at the same iteration
@@ -114,136 +114,7 @@ __global__ void __launch_bounds__(128) hjcd_coarse_kernel(SeedIkArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// coarse phase: eight lanes per seed
-// ---------------------------------------------------------------------------
-
-// For robots of at most 8 joints and 8 actuated joints with one EE.  The
-// descent is a chain of dependent steps over few seeds (256 problems x 32 seeds
-// are 256 warps at one lane per seed, each alone on its scheduler), so a seed
-// gets kCoarseLanes lanes: lane j computes joint j's local transform, the world
-// poses come by pointer doubling along the tree (three rounds of shuffles), lane
-// j builds joint j's Jacobian column and lane c gathers actuated column c, and
-// the best joint is a shuffle reduction.  256 x 32 seeds x 20 steps, with 6
-// refinement iterations after it: 687 -> 598 us.
-constexpr int kCoarseLanes = 8;
-constexpr int kCoarseThreads = 256;
-
-__device__ __forceinline__ Pose shfl_pose(unsigned m, const Pose& T, int from) {
-  return Pose{__shfl_sync(m, T.w, from, kCoarseLanes),  __shfl_sync(m, T.x, from, kCoarseLanes),
-              __shfl_sync(m, T.y, from, kCoarseLanes),  __shfl_sync(m, T.z, from, kCoarseLanes),
-              __shfl_sync(m, T.tx, from, kCoarseLanes), __shfl_sync(m, T.ty, from, kCoarseLanes),
-              __shfl_sync(m, T.tz, from, kCoarseLanes)};
-}
-
-__global__ void __launch_bounds__(kCoarseThreads) hjcd_coarse_lanes_kernel(SeedIkArgs a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int G = kCoarseLanes, NG = kCoarseThreads / G;
-  SeedIkShared& sh = *reinterpret_cast<SeedIkShared*>(smem_raw);
-  RobotSpheresS R = seed_ik_spheres_at(smem_raw + sizeof(SeedIkShared), a.n_rs, a.m.n_joints);
-  float* world = reinterpret_cast<float*>(smem_raw + seed_ik_world_offset(a));
-  float* slots = reinterpret_cast<float*>(smem_raw + seed_ik_slots_offset(a));
-  const int p = blockIdx.y, tid = threadIdx.x, n = a.m.n_act;
-  const int grp = tid / G, gl = tid % G;
-  const unsigned gm = ((1u << G) - 1u) << ((tid & 31) & ~(G - 1));
-  ObsView ob;
-  seed_ik_stage(a, sh, R, world, ob, p, 1);
-  const int s = blockIdx.x * NG + grp;
-  if (s >= a.S) return;  // the whole seed group
-  const size_t gs = (size_t)p * a.S + s;
-  const JointTable& jt = sh.jt;
-  const int nj = jt.n;
-  const bool joint = gl < nj;
-  const int src = joint ? jt.src[gl] : -1, parent = joint ? jt.psorted[gl] : -1;
-  const float mul = joint ? jt.mul[gl] : 0.f, off = joint ? jt.off[gl] : 0.f;
-  const int jk = joint ? jt.jkind[gl] : 0;
-  const float lo = sh.lo[gl], hi = sh.hi[gl];
-  const bool fixed = sh.fixed[gl] != 0;
-  float cfg = gl < n ? a.seeds[gs * n + gl] : 0.f;  // actuated joint gl
-  auto fk = [&]() {
-    const float qv = __shfl_sync(gm, cfg, max(src, 0), G);
-    const float q = (src < 0 ? 0.f : qv) * mul + off;
-    Pose T = joint ? joint_local(jt, gl, q) : pose_identity();
-    int anc = parent;  // T: pose of the joint relative to joint anc's
-#pragma unroll
-    for (int d = 1; d < G; d <<= 1) {
-      const Pose A = shfl_pose(gm, T, max(anc, 0));
-      const int up = __shfl_sync(gm, anc, max(anc, 0), G);
-      if (anc >= 0) {
-        T = pose_compose(A, T);
-        anc = up;
-      }
-    }
-    return T;
-  };
-  float r[6];
-  for (int it = 0; it < a.iters; ++it) {
-    const Pose T = fk();
-    const Pose E = shfl_pose(gm, T, sh.tsorted[0]);
-    seed_ik_pose_error(E, sh.tgt[0][0], r);
-    // adaptive row weights, orientation gated off 1 mm or more from the target
-    const float pn = sqrtf(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]);
-    const float on = sqrtf(r[3] * r[3] + r[4] * r[4] + r[5] * r[5]);
-    float wo = clampf((pn + 1e-8f) / (on + 1e-8f), 0.05f, 1.f);
-    if (pn >= 1e-3f) wo = 0.f;
-    // lane j: joint j's column
-    float col[6];
-    const float3 z = joint ? quat_rotate(T.w, T.x, T.y, T.z, make_float3(jt.axis[gl][0], jt.axis[gl][1], jt.axis[gl][2]))
-                           : make_float3(0.f, 0.f, 0.f);
-    if (jk == 1) {
-      const float ax = E.tx - T.tx, ay = E.ty - T.ty, az = E.tz - T.tz;
-      col[0] = z.y * az - z.z * ay; col[1] = z.z * ax - z.x * az; col[2] = z.x * ay - z.y * ax;
-      col[3] = z.x; col[4] = z.y; col[5] = z.z;
-    } else {
-      col[0] = z.x; col[1] = z.y; col[2] = z.z; col[3] = col[4] = col[5] = 0.f;
-    }
-    // lane c: actuated column c, summed over the joints it drives
-    float J[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int j = 0; j < nj; ++j) {
-      const int a1 = jt.a1[j], a2 = jt.a2[j];
-      if (jt.jkind[j] == 0 || (a1 < 0 && a2 < 0) || !((sh.anc[0] >> jt.orig[j]) & 1ull)) continue;  // uniform
-      const float sm = jt.mul[j];
-      const float wsel = ((gl == a1) ? sm : 0.f) + ((gl == a2) ? sm : 0.f);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) J[k] += wsel * __shfl_sync(gm, col[k], j, G);
-    }
-    float dot = 0.f, sq = 0.f;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      const float wk = k < 3 ? 1.f : wo;
-      const float jw = J[k] * wk;
-      dot += jw * (r[k] * wk);
-      sq += jw * jw;
-    }
-    sq += 1e-8f;
-    // the free joint with the largest predicted decrease, ties to the lowest
-    float impr = dot * dot / sq;
-    if (fixed || !(impr > -1.f)) impr = -1.f;
-    float step = -dot / sq;
-    int best = gl;
-#pragma unroll
-    for (int o = 1; o < G; o <<= 1) {
-      const float oi = __shfl_xor_sync(gm, impr, o), os = __shfl_xor_sync(gm, step, o);
-      const int oc = __shfl_xor_sync(gm, best, o);
-      if (oi > impr || (oi == impr && oc < best)) { impr = oi; step = os; best = oc; }
-    }
-    if (!(impr > -1.f)) break;  // nothing free
-    if (gl == best) cfg = clampf(cfg + step, lo, hi);
-  }
-  const Pose T = fk();
-  const PoseSlots ps{slots + grp, NG};
-  if (joint) ps.store(gl, T);
-  __syncwarp(gm);
-  seed_ik_pose_error(shfl_pose(gm, T, sh.tsorted[0]), sh.tgt[0][0], r);
-  float err = 0.f;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) err += r[k] * r[k];
-  err += seed_ik_penalty<G>(a, ps, R, ob, gl, gm);
-  if (gl == 0) a.out_err[gs] = err;
-  if (gl < n) a.out[gs * n + gl] = cfg;
-}
-
-// ---------------------------------------------------------------------------
-// refinement: one block per problem, four lanes per seed
+// refinement: one warp per problem, one lane per seed
 // ---------------------------------------------------------------------------
 
 // Unweighted squared error plus penalty at the joint poses in `ps`.
@@ -485,22 +356,14 @@ extern "C" int pk_hjcd_ik_coarse_cuda(void* stream, const float* seeds, const fl
   a.enable_collision = enable_collision ? 1 : 0;
   a.collision_weight = collision_weight;
   a.collision_margin = collision_margin;
-  const bool lanes = n_act <= kCoarseLanes && n_joints >= 1 && n_joints <= kCoarseLanes && n_ee == 1;
-  constexpr int kSeedsPerBlock = kCoarseThreads / kCoarseLanes;  // one set of pose slots each
-  const int nth = lanes ? kSeedsPerBlock : n_seeds < 128 ? ((n_seeds + 31) / 32) * 32 : 128;
+  const int nth = n_seeds < 128 ? ((n_seeds + 31) / 32) * 32 : 128;
   size_t smem = 0;
   if (int s = seed_ik_common(a, n_act, n_joints, n_ee, nth < 32 ? 32 : nth, &smem)) return s;
   if (n_problems == 0 || n_seeds == 0) return PK_OK;
   if (int s = seed_ik_check_buffers(a)) return s;
   cudaStream_t st = (cudaStream_t)stream;
-  if (lanes) {
-    if (int s = set_smem_limit((const void*)hjcd_coarse_lanes_kernel, smem)) return s;
-    const dim3 grid((unsigned)((n_seeds + kSeedsPerBlock - 1) / kSeedsPerBlock), (unsigned)n_problems);
-    hjcd_coarse_lanes_kernel<<<grid, kCoarseThreads, smem, st>>>(a);
-    return cuda_status(cudaGetLastError(), "hjcd_coarse_lanes_kernel launch");
-  }
   const int t = nth < 32 ? 32 : nth;
-  if (n_act <= 8 && n_ee == 1) return launch_coarse<8, 1>(a, t, smem, st);  // more than 8 joints
+  if (n_act <= 8 && n_ee == 1) return launch_coarse<8, 1>(a, t, smem, st);
   if (n_ee <= 2) return launch_coarse<16, 2>(a, t, smem, st);
   return launch_coarse<16, 4>(a, t, smem, st);
 }

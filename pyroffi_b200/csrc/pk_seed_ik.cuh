@@ -219,27 +219,8 @@ __device__ inline void seed_ik_stage(const SeedIkArgs& a, SeedIkShared& sh, Robo
   }
 }
 
-// Residual of EE pose T against target pose g (wxyz_xyz): world position
-// difference and the rotation vector of q_ee conj(q_tgt) (w >= 0; 2 v below
-// |v| = 1e-6).
-__device__ __forceinline__ void seed_ik_pose_error(const Pose& T, const float* g, float* r) {
-  r[0] = T.tx - g[4];
-  r[1] = T.ty - g[5];
-  r[2] = T.tz - g[6];
-  const float bw = g[0], bx = -g[1], by = -g[2], bz = -g[3];
-  float qw = T.w * bw - T.x * bx - T.y * by - T.z * bz;
-  float qx = T.w * bx + T.x * bw + T.y * bz - T.z * by;
-  float qy = T.w * by - T.x * bz + T.y * bw + T.z * bx;
-  float qz = T.w * bz + T.x * by - T.y * bx + T.z * bw;
-  if (qw < 0.f) { qw = -qw; qx = -qx; qy = -qy; qz = -qz; }
-  const float s = sqrtf(qx * qx + qy * qy + qz * qz);
-  const float f = s > 1e-6f ? 2.f * atan2f(s, qw) / s : 2.f;
-  r[3] = qx * f;
-  r[4] = qy * f;
-  r[5] = qz * f;
-}
-
-// Residual of every EE against target slot `w`.
+// Residual of every EE against target slot `w`: world position difference and
+// the rotation vector of q_ee conj(q_tgt) (w >= 0; 2 v below |v| = 1e-6).
 template <int MAXEE>
 __device__ __forceinline__ void seed_ik_residual(const SeedIkShared& sh, const PoseSlots& ps, int n_ee, int w,
                                               float (&r)[6 * MAXEE], float (&pee)[3 * MAXEE]) {
@@ -252,7 +233,21 @@ __device__ __forceinline__ void seed_ik_residual(const SeedIkShared& sh, const P
       continue;
     }
     const Pose T = ps.load(sh.tsorted[e]);
-    seed_ik_pose_error(T, sh.tgt[w][e], r + 6 * e);
+    const float* g = sh.tgt[w][e];
+    r[6 * e + 0] = T.tx - g[4];
+    r[6 * e + 1] = T.ty - g[5];
+    r[6 * e + 2] = T.tz - g[6];
+    const float bw = g[0], bx = -g[1], by = -g[2], bz = -g[3];
+    float qw = T.w * bw - T.x * bx - T.y * by - T.z * bz;
+    float qx = T.w * bx + T.x * bw + T.y * bz - T.z * by;
+    float qy = T.w * by - T.x * bz + T.y * bw + T.z * bx;
+    float qz = T.w * bz + T.x * by - T.y * bx + T.z * bw;
+    if (qw < 0.f) { qw = -qw; qx = -qx; qy = -qy; qz = -qz; }
+    const float s = sqrtf(qx * qx + qy * qy + qz * qz);
+    const float f = s > 1e-6f ? 2.f * atan2f(s, qw) / s : 2.f;
+    r[6 * e + 3] = qx * f;
+    r[6 * e + 4] = qy * f;
+    r[6 * e + 5] = qz * f;
     pee[3 * e] = T.tx; pee[3 * e + 1] = T.ty; pee[3 * e + 2] = T.tz;
   }
 }

@@ -117,9 +117,8 @@ def odd_robot(n_joints):
 
 @pytest.mark.parametrize("n_joints", [1, 3, 5, 8, 9])
 @pytest.mark.parametrize("S", [1, 31, 33])
-def test_coarse_lanes_on_trees(n_joints, S):
-    """The eight-lane coarse kernel (up to 8 joints; 9 take the other one) against the FP64 oracle: trees,
-    prismatic, fixed and mimic joints, partial blocks.  A near-tie of two joints may go the other way."""
+def test_coarse_on_trees(n_joints, S):
+    """The coarse kernel against the FP64 oracle: trees, prismatic, fixed and mimic joints, partial blocks.  A near-tie of two joints may go the other way."""
     m = odd_robot(n_joints)
     rng = np.random.default_rng(S)
     link = m.n_links - 1
