@@ -39,8 +39,8 @@ _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def stream_ptr(device: torch.device) -> int:
-    if _raw_stream is None:
-        return torch.cuda.current_stream(device).cuda_stream
+    if _raw_stream is None or type(device) is not torch.device or device.type != "cuda":
+        return torch.cuda.current_stream(device).cuda_stream  # raises for a device without streams
     index = device.index
     return _raw_stream(torch.cuda.current_device() if index is None else index)
 

@@ -190,3 +190,21 @@ def test_nvtx_ranges_wrap_calls_when_asked(monkeypatch):
     monkeypatch.setattr(torch.cuda.nvtx, "range_pop", lambda: pushed.append("pop"))
     _lib.call("pk_chomp_line_select", None, None, None, None, None, None, None, 1, 0.0, 1, 0, 4, 7)
     assert pushed == ["pk_chomp_line_select", "pop"]
+
+
+def test_stream_of_a_device_without_streams_is_refused(monkeypatch):
+    """The raw stream handle is for CUDA devices: any other device still goes to torch, which refuses it."""
+    import torch
+
+    from pyroffi_b200 import _tensors
+
+    def refuse(device):
+        raise ValueError(f"Expected a cuda device, but got: {device}")
+
+    monkeypatch.setattr(_tensors, "_raw_stream", lambda index: 7)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "current_stream", refuse)
+    assert _tensors.stream_ptr(torch.device("cuda", 0)) == 7
+    assert _tensors.stream_ptr(torch.device("cuda")) == 7
+    with pytest.raises(ValueError):
+        _tensors.stream_ptr(torch.device("cpu"))
