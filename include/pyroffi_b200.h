@@ -143,8 +143,9 @@ typedef struct pk_lm_options {
   int32_t enable_collision;
   float collision_weight;
   float collision_margin;
-  int32_t threads_per_seed; /* 0 = default (1 lane; 128 seeds per block up to 8 DOF / 1 EE, 96 up to 16 DOF /
-                              2 EEs); 1, 2, 4, 8 = lanes sharing one seed; 5 = one lane per line-search
+  int32_t threads_per_seed; /* 0 = default (1 lane, and up to 8 DOF / 1 EE a second one for the line-search
+                              trials where two such blocks fit an SM; 128 seeds per block up to 8 DOF / 1 EE,
+                              96 up to 16 DOF / 2 EEs); 1, 2, 4, 8 = lanes sharing one seed; 5 = one lane per line-search
                               trial; 16, 32 = warp-per-seed body with that many lanes per seed */
   int32_t seeds_per_block;  /* 0 = choose automatically */
   int32_t lanes_per_wide_seed; /* warp-per-seed body: lanes per seed, 16 (0 = default) or 32 */
@@ -244,7 +245,8 @@ typedef struct pk_ik_class {
  * one persistent kernel whose blocks take items from a device counter in
  * queue[2] (caller-owned device memory; cleared here with async memsets on
  * `stream` before the launches, so one queue serves one call in flight at
- * a time; bodies 0 and 2 use queue[0] one after the other).  blocks = 0
+ * a time; bodies 0 and 2 share queue[0], 16 bits each, or from 65,536 items
+ * and blocks on one after the other).  blocks = 0
  * sizes each grid to one full wave on the current device.  Same per-seed
  * iteration and outputs as pk_ls_ik_ex with opt.
  */

@@ -150,8 +150,7 @@ __host__ __device__ inline size_t lm_align16(size_t x) { return (x + 15) & ~size
 // spheres in pairs (float4 (x0, x1, y0, y1), (z0, z1, r0, r1); an odd joint
 // padded with a sphere of radius -1e9), and each self-pair group's pairs in
 // pairs (float4 (-ax0, -ax1, -ay0, -ay1), (-az0, -az1, rr0, rr1),
-// (bx0, bx1, by0, by1), (bz0, bz1, rr0|rr0|, rr1|rr1|) with rr = r_a + r_b +
-// margin; an odd group padded with a pair that never hits).  The staging
+// (bx0, bx1, by0, by1), (bz0, bz1, 0, 0) with rr = r_a + r_b + margin; an odd group padded with a pair that never hits).  The staging
 // scratch (self-pair key counts, obstacle boxes) overlays the per-seed area
 // before the seeds run.
 // threads > 0: trial-lane kernel (per-lane pose slots for `threads` lanes,
@@ -281,7 +280,8 @@ __device__ __forceinline__ void hinge_sq(float d2, float rr, float& pen) {
 // Exact hinge terms of the sphere pairs [p0, p1) of a joint against world
 // sphere O (radius already + margin), with the obstacle centre moved into
 // the joint's frame (T: the joint's rotation and its bounding centre, jb) once: |R c_k + t - o| = |c_k - R^T (o - t)|; two
-// spheres per packed FP32x2 operation, terms added in sphere order.
+// spheres per packed FP32x2 operation (the even and the odd spheres' terms add
+// up apart).
 __device__ __forceinline__ void narrow_world(const PenaltyCtx& c, const Pose& T, float4 jb, int p0, int p1, float4 O,
                                              float& pen) {
   float3 o = pose_apply_inv(T, make_float3(O.x, O.y, O.z));  // relative to the bounding centre
@@ -304,7 +304,7 @@ __device__ __forceinline__ void narrow_world(const PenaltyCtx& c, const Pose& T,
 }
 
 // Hinge terms of the pairs of self-pair group gi of one seed (poses in ps),
-// added to pen in pair order: one relative transform T_x^-1 T_y (rotation
+// added to pen (the even and the odd pairs' terms add up apart): one relative transform T_x^-1 T_y (rotation
 // conj(q_x) q_y as a matrix M, translation u = R_x^T (t_y - t_x)), then per
 // pair |c_a - (M c_b + u)| from the joint-frame records, two pairs per
 // packed FP32x2 operation.
@@ -1123,10 +1123,10 @@ __device__ void lm_stage(const LmArgs& a, unsigned char* smem_raw, const LmLayou
             const float4 A = rs4[pr.x], Bs = rs4[pr.y];
             const float rr = A.w + Bs.w + a.margin;
             f[h] = -A.x; f[2 + h] = -A.y; f[4 + h] = -A.z; f[6 + h] = rr;
-            f[8 + h] = Bs.x; f[10 + h] = Bs.y; f[12 + h] = Bs.z; f[14 + h] = rr * fabsf(rr);
-          } else {  // padding: |u|^2 >= 0 is never below -1
+            f[8 + h] = Bs.x; f[10 + h] = Bs.y; f[12 + h] = Bs.z; f[14 + h] = 0.f;
+          } else {  // padding: a radius sum of -1 never hits
             f[h] = 0.f; f[2 + h] = 0.f; f[4 + h] = 0.f; f[6 + h] = -1.f;
-            f[8 + h] = 0.f; f[10 + h] = 0.f; f[12 + h] = 0.f; f[14 + h] = -1.f;
+            f[8 + h] = 0.f; f[10 + h] = 0.f; f[12 + h] = 0.f; f[14 + h] = 0.f;
           }
         }
       }

@@ -221,3 +221,26 @@ def test_sphere_count_variants_match_oracle(per_link):
     np.testing.assert_allclose(c.cpu().numpy(), osco.coll_sum(q, *oracle_args(w), 0.01, True), rtol=1e-5, atol=1e-6)
     oJ = osco.group_jacobian(q, *oracle_args(w), TAU, True, eps=1e-6)
     np.testing.assert_allclose(J.cpu().numpy(), oJ, atol=2e-4, rtol=1e-3)
+
+
+def test_smaller_blocks_for_a_world_that_fills_shared_memory():
+    """Spheres out of reach pad the world to the most that is accepted, which leaves room for the placed link
+    spheres of fewer waypoints per block: distances and Jacobians as without the padding, whose softmax
+    weights are exp(-2000)."""
+    from pyroffi_b200._lib import PkError
+    w = W.mixed_trajectories(Bt=3, T=8, per_link=20)
+    q = torch.as_tensor(w.traj.reshape(-1, w.traj.shape[-1]), device=DEV)
+    d0, J0, _ = make(w).linearize(q)
+    near = w.world.spheres
+    for total in range(14336, 8192, -64):
+        w.world.spheres = np.concatenate([near, np.tile(np.array([[100.0, 0, 0, 0.1]], np.float32),
+                                                        (total - len(near), 1))])
+        try:
+            d, J, _ = make(w).linearize(q)
+            break
+        except PkError:  # refused on the host: too much for shared memory
+            continue
+    else:
+        pytest.fail("no padded world was accepted")
+    np.testing.assert_allclose(d.cpu().numpy(), d0.cpu().numpy(), rtol=1e-6, atol=1e-6)
+    np.testing.assert_allclose(J.cpu().numpy(), J0.cpu().numpy(), rtol=1e-5, atol=1e-6)

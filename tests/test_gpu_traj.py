@@ -53,6 +53,30 @@ def test_cost_over_obstacle_chunks(Ms):
     np.testing.assert_allclose(c, ref, rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("n", [1, 31, 33, 65])
+def test_listed_capsules_and_boxes(n):
+    """A warp lists the capsules and boxes near its waypoints 32 at a time by their bounding spheres: counts
+    around one and two rounds, long thin ones among them, some out of reach and some not; the cost of the
+    launch without a gradient and of the one with it."""
+    rng = np.random.default_rng(n)
+    w, _ = setup(Bt=2, T=9)
+    a = rng.uniform(-1.0, 1.0, (n, 3))
+    u = rng.normal(size=(n, 3))
+    u /= np.linalg.norm(u, axis=1, keepdims=True)
+    w.world.capsules = np.concatenate([a, a + rng.uniform(0.0, 2.0, (n, 1)) * u, rng.uniform(0.01, 0.1, (n, 1))],
+                                      axis=1).astype(np.float32)
+    axes = np.linalg.qr(rng.normal(size=(n, 3, 3)))[0]
+    w.world.boxes = np.concatenate([rng.uniform(-1.5, 1.5, (n, 3)), axes.transpose(0, 2, 1).reshape(n, 9),
+                                    rng.uniform(0.01, 0.7, (n, 3))], axis=1).astype(np.float32)
+    tc = TrajectoryCost(w.model, w.spheres, w.world, w.link_pairs, margin=w.margin, w_smooth=0.0, w_acc=0.0,
+                        w_jerk=0.0, w_limits=0.0, w_coll=1.0, device=DEV)
+    x = torch.as_tensor(w.traj, device=DEV)
+    ref = np.array([otr.collision_cost(w.traj[b], w.model.as_dict(), w.spheres.centers, w.spheres.radii, w.link_pairs,
+                                       w.world.arrays(), w.margin) for b in range(2)])
+    np.testing.assert_allclose(tc.cost(x).cpu().numpy(), ref, rtol=1e-4, atol=1e-5)
+    np.testing.assert_allclose(tc.cost_and_grad(x)[0].cpu().numpy(), ref, rtol=1e-4, atol=1e-5)
+
+
 def test_gradient_matches_finite_differences():
     w, tc = setup(Bt=3, T=12)
     x = torch.as_tensor(w.traj, device=DEV)
