@@ -43,17 +43,16 @@ P_PER_GPU, SEEDS, ITERS = 256, 128, 30
 FLOP_PER_SEED_ITER = 6 * (130 * 7 + 60 + 33 * 56 + 12 * 56 * 100 + 12 * 200) + 45 * 7 + 800
 L2_FLUSH_BYTES = 256 << 20
 # From one ncu capture of one launch of the LM kernel on this workload (python -m
-# pyroffi_b200.profile_cases lm): DRAM bytes read + written (the ~1 MB of outputs were still in L2
-# when the launch ended), and the FP32 work the kernel executed, 2 FLOP per FFMA, 1 per FADD / FMUL,
+# pyroffi_b200.profile_cases lm): DRAM bytes read + written, and the FP32 work the kernel executed, 2 FLOP per FFMA, 1 per FADD / FMUL,
 # twice that for the packed FFMA2 / FADD2 / FMUL2, summed over threads; the FMA pipe's active share.
-LM_DRAM_BYTES_PER_LAUNCH = 1087744 + 256
-LM_EXECUTED_FLOP_PER_LAUNCH = 29031424050
-LM_FMA_PIPE_PCT = 15.5
+LM_DRAM_BYTES_PER_LAUNCH = 1132544 + 1087232
+LM_EXECUTED_FLOP_PER_LAUNCH = 39087924997
+LM_FMA_PIPE_PCT = 32.5
 # The same counts for the trajectory kernel's fused forward + backward launch on the 512 x 64 x 7 workload
 # (python -m pyroffi_b200.profile_cases traj) and for the fused FK + collision kernel on the sweep robot's
 # per-link rows (python -m pyroffi_b200.profile_cases fkc5, 4,096 configurations; per configuration).
-TRAJ_EXECUTED_FLOP_PER_LAUNCH = 1339234465
-TRAJ_FMA_PIPE_PCT = 29.9
+TRAJ_EXECUTED_FLOP_PER_LAUNCH = 614165205
+TRAJ_FMA_PIPE_PCT = 23.3
 SWEEP_EXECUTED_FLOP_PER_CONFIG = 27802706944 / 4096
 SWEEP_FMA_PIPE_PCT = 60.4
 
