@@ -64,6 +64,9 @@ __device__ __forceinline__ float4 box_ball(const float* b) {
 // Obstacles that a warp's candidate list has room for: all but the halfspaces.
 __host__ __device__ __forceinline__ int listed(const WorldArgs& w) { return w.Ms + w.Mc + w.Mb; }
 
+// Warps of a block; two lanes for each of up to 8 waypoints are half a warp.
+__host__ __device__ __forceinline__ int traj_warps(int nth) { return (nth + 31) >> 5; }
+
 // Lanes per waypoint: the world (link, obstacle) pairs and the self pairs of
 // one waypoint are split over a group of TG lanes (TG = 2 or 4); its FK,
 // force totals and joint gradient live once per waypoint in shared memory.
@@ -91,7 +94,7 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
   float* lt = reinterpret_cast<float*>(p); p += sizeof(float) * N * 6 * ng;       // link force / moment totals
   float* gq = reinterpret_cast<float*>(p); p += sizeof(float) * nj * ng;          // gradient per joint
   unsigned short* cand = reinterpret_cast<unsigned short*>(p) + (size_t)(tid >> 5) * listed(a.w);  // this warp's candidates
-  if (a.list) p += sizeof(unsigned short) * (size_t)listed(a.w) * (nth >> 5);
+  if (a.list) p += sizeof(unsigned short) * (size_t)listed(a.w) * traj_warps(nth);
   p = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15));
 
   load_joint_table(jt, a.m);
@@ -132,9 +135,10 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
 
   constexpr bool want_grad = GRAD;
   const float margin = a.margin;
+  const unsigned lanes = nth < 32 ? (1u << nth) - 1u : 0xffffffffu;  // of every warp of the block
   for (int t0 = 0; t0 < T; t0 += ng) {
     const int t = t0 + grp;
-    const unsigned wm = __ballot_sync(0xffffffffu, t < T);  // the warp's lanes at work: a prefix of it
+    const unsigned wm = __ballot_sync(lanes, t < T);  // the warp's lanes at work: a prefix of it
     if (t >= T) continue;  // the whole group skips
     const PoseSlots ps{slots + grp, ng};
     if (gl == 0) fk_thread(jt, [&](int i) { return xs[t * n + i]; }, ps);
@@ -427,7 +431,7 @@ static size_t traj_smem(const TrajArgs& a, int nth, int TG) {
              2 * sizeof(float) * ((a.T * a.m.n_act + 3) & ~3) + sizeof(float) * ((nth + 3) & ~3) +
              sizeof(float) * ((a.T + 3) & ~3) +
              sizeof(float) * (size_t)(nth / TG) * (a.m.n_joints * 7 + a.N * 6 + a.m.n_joints) +
-             (a.list ? sizeof(unsigned short) * (size_t)listed(a.w) * (nth / 32) : 0);
+             (a.list ? sizeof(unsigned short) * (size_t)listed(a.w) * traj_warps(nth) : 0);
   s = (s + 15) & ~size_t(15);
   return s + sizeof(float) * a.w.smem_floats();
 }

@@ -176,6 +176,33 @@ def test_large_batch_two_lane_path_matches_oracle():
         assert rel < 1e-4, (b, rel)
 
 
+@pytest.mark.parametrize("T", [5, 8, 9])
+@pytest.mark.parametrize("n_spheres", [3, 65])
+def test_short_trajectories_in_large_batches(T, n_spheres):
+    """Two lanes for each of up to 8 waypoints make blocks of half a warp (9: a whole one), whose candidate
+    list needs its own shared memory: cost and gradient of a large batch as of its parts, which take four
+    lanes, and as the oracle's.  All obstacles are within reach of the arm, capsules and boxes among them."""
+    rng = np.random.default_rng(T)
+    w = W.trajectories(Bt=320, T=T)
+    w.world.spheres = W.random_sphere_world(rng, n_spheres, lo=-0.5, hi=0.5)
+    w.world.capsules = W.random_capsules(rng, 7)
+    w.world.boxes = W.random_boxes(rng, 5, oriented=True)
+    tc = TrajectoryCost(w.model, w.spheres, w.world, w.link_pairs, margin=w.margin, w_smooth=0.0, w_acc=0.0,
+                        w_jerk=0.0, w_limits=0.0, w_coll=1.0, device=DEV)
+    x = torch.as_tensor(w.traj, device=DEV)
+    c, g = (v.cpu().numpy() for v in tc.cost_and_grad(x))
+    np.testing.assert_array_equal(tc.cost(x).cpu().numpy(), c)
+    part = [tc.cost_and_grad(x[i:i + 160].contiguous()) for i in (0, 160)]
+    np.testing.assert_allclose(c, torch.cat([v[0] for v in part]).cpu().numpy(), rtol=1e-5, atol=1e-6)
+    np.testing.assert_allclose(g, torch.cat([v[1] for v in part]).cpu().numpy(), rtol=1e-4, atol=1e-4)
+    args = (w.model.as_dict(), w.spheres.centers, w.spheres.radii, w.link_pairs, w.world.arrays(), w.margin)
+    ref = np.array([otr.collision_cost(w.traj[b].astype(np.float64), *args) for b in range(0, 320, 16)])
+    np.testing.assert_allclose(c[::16], ref, rtol=1e-4, atol=1e-5)
+    b = int(np.argmax(c))
+    ref = otr.collision_grad_fd(w.traj[b].astype(np.float64), *args)
+    assert np.linalg.norm(g[b] - ref) / np.linalg.norm(ref) < 1e-4
+
+
 @pytest.mark.parametrize("per_link", [8, 16, 20])
 def test_sphere_count_variants_match_oracle(per_link):
     """Kernels for up to 8, 16 and 32 spheres per link (register pairs)."""
