@@ -545,6 +545,7 @@ __global__ void __launch_bounds__(128, MAXS <= 8 ? 4 : (MAXS <= 16 ? 3 : 2)) sco
 #pragma unroll
         for (int g = 0; g < kScoG; ++g) gref[g] = __shfl_sync(gm, rg, lane0 + g);
       }
+      __syncwarp(gm);  // the next link's spheres go in the same place
     }
     if (a.coll) {
       csum = group_sum<TG>(csum, gm);

@@ -133,6 +133,28 @@ def test_final_cost_matches_oracle():
         np.testing.assert_allclose(c[b], oc, rtol=2e-5)
 
 
+def test_collision_sum_with_uneven_lanes():
+    """The lanes of a waypoint share one copy of a link's spheres.  With the obstacles near the arm all in
+    lane 0's share (every eighth) the other lanes are done with a link long before it is: the collision sums
+    and costs as the oracle's, and the same bits each time."""
+    w = scene(Bt=64, T=12)
+    near = W.random_sphere_world(np.random.default_rng(2), 40, lo=-0.5, hi=0.5)
+    w.world.spheres = np.tile(np.array([[50.0, 0, 0, 0.1]], np.float32), (8 * len(near), 1))
+    w.world.spheres[::8] = near
+    opt = make(w)
+    x = torch.as_tensor(w.traj, device=DEV)
+    q = x.reshape(-1, x.shape[-1])
+    first = opt.final_cost(x), opt.linearize(q, want_jac=False, want_coll=True)[2]
+    for _ in range(5):
+        assert torch.equal(opt.final_cost(x), first[0])
+        assert torch.equal(opt.linearize(q, want_jac=False, want_coll=True)[2], first[1])
+    np.testing.assert_allclose(first[1][:48].cpu().numpy(),
+                               osco.coll_sum(w.traj[:4].reshape(48, -1), *oracle_args(w), 0.01, True), rtol=1e-5, atol=1e-6)
+    for b in range(4):
+        np.testing.assert_allclose(float(first[0][b]), osco.ranking_cost(w.traj[b], *oracle_args(w), w.model.lower,
+                                                                         w.model.upper, ScoConfig()), rtol=2e-5)
+
+
 @pytest.mark.parametrize("fd_eps", [0.0, 1e-4])
 def test_single_call_equals_staged_calls(fd_eps):
     w = scene()
