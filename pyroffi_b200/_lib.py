@@ -145,8 +145,8 @@ def load() -> C.CDLL:
         lib.pk_version.restype = C.c_char_p
         lib.pk_status_string.restype = C.c_char_p
         lib.pk_status_string.argtypes = [C.c_int]
-        _fns.update(fns)
         _lib = lib
+        _fns.update(fns)  # last: call() takes a function from here without the lock and then relies on _lib
         return lib
 
 

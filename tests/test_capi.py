@@ -208,3 +208,20 @@ def test_stream_of_a_device_without_streams_is_refused(monkeypatch):
     assert _tensors.stream_ptr(torch.device("cuda")) == 7
     with pytest.raises(ValueError):
         _tensors.stream_ptr(torch.device("cpu"))
+
+
+def test_functions_are_published_after_the_library(monkeypatch):
+    """A thread that finds its function while another one is still in load() can report the call's error."""
+    statuses = []
+
+    class Published(dict):
+        def update(self, fns):
+            super().update(fns)
+            with pytest.raises(_lib.PkError, match="negative batch"):  # what another thread may do from here on
+                _lib.call("pk_fk_cuda", *([None] * 13), -1, 7, 7, 7)
+            statuses.append("reported")
+
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib, "_fns", Published())
+    _lib.load()
+    assert statuses == ["reported"]
