@@ -467,6 +467,7 @@ __device__ float penalty_share(const PenaltyCtx& c, const PoseSlots& ps, int t, 
   float pen = 0.f;
   const bool b4 = B4;
   if (need) {
+    if (TPS > 1) __syncwarp(gmask);  // the seed's other lanes have read the positions (residual) that go
     for (int j = t; j < c.n_js; j += TPS) {
       const int js = c.jlist[j];
       const float4 bl = c.jb[j];

@@ -32,7 +32,8 @@ def mixed_world(rng):
     return w
 
 
-@pytest.mark.parametrize("robot,tps", [("chain7", 2), ("chain7", 4), ("chain7", 16), ("bimanual", 16), ("bimanual", 32)])
+@pytest.mark.parametrize("robot,tps", [("chain7", 0), ("chain7", 1), ("chain7", 2), ("chain7", 4), ("chain7", 8),
+                                       ("chain7", 16), ("bimanual", 16), ("bimanual", 32)])
 @pytest.mark.parametrize("max_iter", [0, 1, 2])
 def test_lm_mixed_world_and_self_pairs(robot, tps, max_iter):
     rng = np.random.default_rng(21)
@@ -58,6 +59,8 @@ def test_lm_mixed_world_and_self_pairs(robot, tps, max_iter):
     s = BatchIkSolver(model, links, spheres=spheres, world=world, self_pairs=pairs, threads_per_seed=tps,
                       device=DEV, **opts)
     cfgs, errs = s.run_lm(tt(target), tt(seeds))
+    again = s.run_lm(tt(target), tt(seeds))  # the lanes of a seed share its poses: the same bits each time
+    assert torch.equal(again[0], cfgs) and torch.equal(again[1], errs)
     cfgs, errs = cfgs.cpu().numpy(), errs.cpu().numpy()
     ok = 0
     for p in range(P):
