@@ -14,6 +14,8 @@
 // arithmetic.  Both are bound by FP32 issue and the reciprocal square roots
 // (one per sphere-obstacle or sphere-sphere pair), and take one Newton step on
 // the root so the distances keep the accuracy of the IEEE square root.
+#include <algorithm>
+
 #include "pk_obstacles.cuh"
 
 namespace pk {
@@ -535,11 +537,15 @@ extern "C" int pk_collision_world_sphere_reduced(void* stream, const float* cent
   const bool aligned = w.spheres == nullptr || (reinterpret_cast<uintptr_t>(w.spheres) & 15) == 0;
   r.stage = wbytes <= 48 * 1024 || (!aligned && wbytes <= kWorldSmemLimit);
   const size_t wsm = r.stage ? wbytes : 0;
-  if (link_rows_smem(1, r.N, r.S) + wsm <= 200 * 1024 && (r.stage || aligned)) {
+  // a block counts its (row, obstacle) pairs of a kind (quads, for spheres) in
+  // 32 bits, with room for the step past the last one
+  const long long most = (1LL << 31) - 1024, wide = std::max({(Ms + 3LL) / 4, (long long)Mc, (long long)Mb, (long long)Mh});
+  if (link_rows_smem(1, r.N, r.S) + wsm <= 200 * 1024 && (r.stage || aligned) && n * wide <= most) {
     // as many configurations per block (at most 8) as leave three blocks for
     // every SM and fit half of its shared memory
     r.cpb = 8;
-    while (r.cpb > 1 && ((B + r.cpb - 1) / r.cpb < 3 * 148 || link_rows_smem(r.cpb, r.N, r.S) + wsm > 100 * 1024))
+    while (r.cpb > 1 && ((B + r.cpb - 1) / r.cpb < 3 * 148 || link_rows_smem(r.cpb, r.N, r.S) + wsm > 100 * 1024 ||
+                         r.cpb * n * wide > most))
       r.cpb >>= 1;
     const size_t smem = link_rows_smem(r.cpb, r.N, r.S) + wsm;
     const long long blocks = (B + r.cpb - 1) / r.cpb;

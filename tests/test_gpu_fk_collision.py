@@ -181,6 +181,24 @@ def test_packed_links_with_nan_and_infinity():
         np.testing.assert_array_equal(a.cpu().numpy(), b.cpu().numpy())
 
 
+def test_reduced_rows_past_32_bits():
+    """1,024 links against 8.4 million obstacles: more (link, obstacle) pairs than 32 bits count."""
+    N, Ms = 1024, (1 << 23) + 8
+    rng = np.random.default_rng(5)
+    c, r = rng.uniform(-1, 1, (1, N, 3)).astype(np.float32), np.full((1, N), 0.1, np.float32)
+    g = torch.Generator(device=DEV).manual_seed(5)
+    ws = 2.0 * torch.rand((Ms, 4), device=DEV, generator=g) - 1.0
+    world = [ws, *[tt(np.zeros((0, k), np.float32)) for k in (7, 15, 6)]]
+    out = collision_world_sphere_reduced(tt(np.ascontiguousarray(c.transpose(2, 0, 1))), tt(r), *world, n=N)
+    assert out.shape == (1, N, Ms)
+    cols = torch.as_tensor([0, 1, 2, 3, 1000, Ms // 4, Ms // 2, 3 * Ms // 4 + 1, Ms - 2, Ms - 1], device=DEV)
+    w8 = ws[cols].cpu().numpy().astype(np.float64)
+    ref = np.linalg.norm(c[0, :, None].astype(np.float64) - w8[None, :, :3], axis=-1) - r[0, :, None] - w8[None, :, 3]
+    np.testing.assert_allclose(out[0, :, cols].cpu().numpy(), ref, atol=1e-6)
+    del out
+    torch.cuda.empty_cache()
+
+
 def test_world_capsule_robot():
     rng = np.random.default_rng(12)
     B, N = 19, 5
