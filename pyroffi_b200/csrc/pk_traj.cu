@@ -58,7 +58,15 @@ __device__ __forceinline__ float4 capsule_ball(const float* c) {
   return make_float4(c[0] + hx, c[1] + hy, c[2] + hz, c[6] + sqrtf(hx * hx + hy * hy + hz * hz));
 }
 __device__ __forceinline__ float4 box_ball(const float* b) {
-  return make_float4(b[0], b[1], b[2], sqrtf(b[12] * b[12] + b[13] * b[13] + b[14] * b[14]));
+  return make_float4(b[0], b[1], b[2], 1.0001f * sqrtf(b[12] * b[12] + b[13] * b[13] + b[14] * b[14]));
+}
+// Are a box's axes orthonormal to within rounding?  Only then does the ball
+// hold it: a box of axes half as long is twice as large.
+__device__ __forceinline__ bool box_orthonormal(const float* b) {
+  auto dot = [&](int i, int j) { return b[i] * b[j] + b[i + 1] * b[j + 1] + b[i + 2] * b[j + 2]; };
+  const float off = fmaxf(fmaxf(fabsf(dot(3, 6)), fabsf(dot(3, 9))), fabsf(dot(6, 9)));
+  const float len = fmaxf(fmaxf(fabsf(dot(3, 3) - 1.f), fabsf(dot(6, 6) - 1.f)), fabsf(dot(9, 9) - 1.f));
+  return fmaxf(off, len) < 1e-5f;
 }
 
 // Obstacles that a warp's candidate list has room for: all but the halfspaces.
@@ -131,7 +139,9 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
     // R < 0 marks a link without spheres; the slack keeps the cull conservative
     lbnd[l] = cnt ? make_float4(cx, cy, cz, R + 1e-4f + 1e-5f * fabsf(R)) : make_float4(0.f, 0.f, 0.f, -1.f);
   }
-  __syncthreads();
+  bool balls = true;
+  for (int k = tid; k < ob.Mb; k += nth) balls = balls && box_orthonormal(ob.box + 15 * k);
+  const bool list_boxes = __syncthreads_and(balls) && a.list;  // else every box is tested
 
   constexpr bool want_grad = GRAD;
   const float margin = a.margin;
@@ -222,8 +232,8 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
       const int lane = tid & 31, step = __popc(wm);
       int n_cand = 0;
       // lists obstacles base, base + 1, ... (ball(k): the bounding sphere of the k-th); returns their number
-      auto list_kind = [&](int base, int count, auto ball) {
-        if (!a.list) return count;
+      auto list_kind = [&](bool list, int base, int count, auto ball) {
+        if (!list) return count;
         const int first = n_cand;
         for (int k0 = 0; k0 < count; k0 += step) {
           const int k = k0 + lane;
@@ -243,14 +253,14 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
         return n_cand - first;
       };
       const int b1 = ob.Ms, b2 = b1 + ob.Mc, b3 = b2 + ob.Mb;
-      const int n0 = list_kind(0, ob.Ms, [&](int k) { return ob.sph[k]; });
-      const int n1 = list_kind(b1, ob.Mc, [&](int k) { return capsule_ball(ob.cap + 7 * k); });
-      const int n2 = list_kind(b2, ob.Mb, [&](int k) { return box_ball(ob.box + 15 * k); });
+      const int n0 = list_kind(a.list, 0, ob.Ms, [&](int k) { return ob.sph[k]; });
+      const int n1 = list_kind(a.list, b1, ob.Mc, [&](int k) { return capsule_ball(ob.cap + 7 * k); });
+      const int n2 = list_kind(list_boxes, b2, ob.Mb, [&](int k) { return box_ball(ob.box + 15 * k); });
       __syncwarp(wm);
       near_of_kind<0>(ob, [&](int i) { return a.list ? (int)cand[i] : i; }, n0, B, bl.w, margin, gl, TG, narrow);
       near_of_kind<1>(ob, [&](int i) { return a.list ? (int)cand[n0 + i] : b1 + i; }, n1, B, bl.w, margin, gl, TG, narrow);
-      near_of_kind<2>(ob, [&](int i) { return a.list ? (int)cand[n0 + n1 + i] : b2 + i; }, n2, B, bl.w, margin, gl, TG,
-                      narrow);
+      near_of_kind<2>(ob, [&](int i) { return list_boxes ? (int)cand[n0 + n1 + i] : b2 + i; }, n2, B, bl.w, margin, gl,
+                      TG, narrow);
       near_of_kind<3>(ob, [=](int i) { return b3 + i; }, ob.Mh, B, bl.w, margin, gl, TG, narrow);
       __syncwarp(wm);  // the next link's list goes in the same place
       if (want_grad) {

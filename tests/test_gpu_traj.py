@@ -77,6 +77,23 @@ def test_listed_capsules_and_boxes(n):
     np.testing.assert_allclose(tc.cost_and_grad(x)[0].cpu().numpy(), ref, rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("scale", [(0.5, 0.5, 0.5), (1.0, 0.3, 1.0)])
+def test_boxes_with_short_axes(scale):
+    """Axes shorter than 1 stretch a box past its half lengths: none of it may be lost to the list's balls."""
+    rng = np.random.default_rng(8)
+    w, _ = setup(Bt=2, T=9)
+    w.world.spheres = w.world.spheres[:1]
+    w.world.boxes = W.random_boxes(rng, 12, oriented=True)
+    w.world.boxes[:, 3:12] = (w.world.boxes[:, 3:12].reshape(-1, 3, 3) * np.array(scale, np.float32)[:, None]).reshape(-1, 9)
+    tc = TrajectoryCost(w.model, w.spheres, w.world, w.link_pairs, margin=w.margin, w_smooth=0.0, w_acc=0.0,
+                        w_jerk=0.0, w_limits=0.0, w_coll=1.0, device=DEV)
+    x = torch.as_tensor(w.traj, device=DEV)
+    ref = np.array([otr.collision_cost(w.traj[b], w.model.as_dict(), w.spheres.centers, w.spheres.radii, w.link_pairs,
+                                       w.world.arrays(), w.margin) for b in range(2)])
+    np.testing.assert_allclose(tc.cost(x).cpu().numpy(), ref, rtol=1e-4, atol=1e-5)
+    np.testing.assert_allclose(tc.cost_and_grad(x)[0].cpu().numpy(), ref, rtol=1e-4, atol=1e-5)
+
+
 def test_gradient_matches_finite_differences():
     w, tc = setup(Bt=3, T=12)
     x = torch.as_tensor(w.traj, device=DEV)
