@@ -2004,7 +2004,9 @@ static int launch_lm(LmArgs a, int tps, int spb, cudaStream_t st) {
     if (spb <= 0) {
       const bool small = a.n_act <= 8 && a.n_ee <= 1;
       spb = small ? 128 : kSeedsPerBlock16;
-      a.trial_lanes = small && !a.f64_solve ? 2 : 1;
+      // (a trial is skipped when its pose error alone cannot win, which with a
+      // negative weight depends on which trials have been seen)
+      a.trial_lanes = small && !a.f64_solve && !(a.coll && a.coll_w < 0.f) ? 2 : 1;
     }
   }
   if (tps == 5) {

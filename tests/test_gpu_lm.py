@@ -352,3 +352,14 @@ def test_trial_lanes_equal_one_lane(Sd, n_self, iters):
                                                                                                    tt(w.seeds))
     close = ((a[0] - b[0]).abs().amax(-1) < 2e-4) & ((a[1] - b[1]).abs() <= 1e-3 * b[1].abs() + 1e-4)
     assert close.float().mean() >= 0.97
+
+
+def test_negative_collision_weight_takes_one_lane():
+    """With a negative weight the skipped trials depend on the order they are seen in: one lane per seed."""
+    w = W.ik(P=3, Sd=64)
+    kw = dict(spheres=w.spheres, world=w.world, self_pairs=w.self_pairs, max_iter=4, lambda_init=w.lambda_init,
+              lambda_down=w.lambda_down, lambda_up=w.lambda_up, collision_weight=-1e4, device=DEV)
+    a = BatchIkSolver(w.model, w.target_link, **kw).run_lm(tt(w.target_T), tt(w.seeds))
+    b = BatchIkSolver(w.model, w.target_link, threads_per_seed=1, seeds_per_block=128, **kw).run_lm(tt(w.target_T),
+                                                                                                   tt(w.seeds))
+    assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1])
