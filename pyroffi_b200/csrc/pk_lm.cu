@@ -135,6 +135,7 @@ struct LmLayout {
   size_t rs, rsp, ws, pairs, pair4, prec, pgstart, wscr, gjoint, gstart, rsj, rsk, cells, cell_obs, wc, wb, wh, slots, pos, scratch,
       total;
   int ms_pad, grid, max_entries, scratch_ints, recs;
+  int cell_ints;  // place of the grid's int offsets in the scratch (0: that of the offsets themselves)
 };
 
 __host__ __device__ inline size_t lm_align16(size_t x) { return (x + 15) & ~size_t(15); }
@@ -162,8 +163,7 @@ __host__ __device__ inline LmLayout lm_layout(const LmArgs& a, int tps, int thre
   const int nc = a.spb * max(a.trial_lanes, 1);  // configurations in flight
   L.ms_pad = lm_ms_pad(a.w.Ms, tps);
   if (threads == 0) {
-    // obstacle boxes and the grid's offsets as ints while it is built
-    L.scratch_ints = a.coll ? max(a.m.n_joints, a.w.Ms + 4 + obstacle_grid_cells(a.grid_n) + 1) : 0;
+    L.scratch_ints = a.coll ? max(a.m.n_joints, a.w.Ms) : 0;  // obstacle boxes
   } else {
     L.scratch_ints = 7 * a.m.n_joints * threads;  // the pose slots double as staging scratch
   }
@@ -190,7 +190,24 @@ __host__ __device__ inline LmLayout lm_layout(const LmArgs& a, int tps, int thre
   L.gstart = o; o = lm_align16(o + 4 * (size_t)(n_self + 2));
   L.rsj = o; o = lm_align16(o + 4 * (size_t)n_rs);
   L.rsk = o; o = lm_align16(o + 4 * (size_t)n_rs);
-  L.cells = o; o = lm_align16(o + (L.grid ? (threads == 0 ? 2 : 4) * (size_t)(obstacle_grid_cells(a.grid_n) + 1) : 0));
+  // The grid is built on 32-bit offsets; the seed-group kernels then keep them
+  // in 16.  The ints lie in the scratch while the grid is built, or where that
+  // would take more (few pose slots, many obstacles) in the place of the 16-bit
+  // ones.
+  const size_t offsets = L.grid ? obstacle_grid_cells(a.grid_n) + 1 : 0;
+  L.cell_ints = 0;
+  size_t cell_bytes = 4 * offsets;
+  if (threads == 0 && L.grid) {
+    const size_t slots = 28 * (size_t)a.m.n_joints * nc, boxes = 4 * (size_t)((a.w.Ms + 3) & ~3);
+    const size_t apart = lm_align16(2 * offsets) + max(slots, boxes + 4 * offsets);
+    const size_t in_place = lm_align16(4 * offsets) + max(slots, 4 * (size_t)L.scratch_ints);
+    if (apart <= in_place) {
+      L.cell_ints = boxes / 4;
+      L.scratch_ints = max(L.scratch_ints, (int)(boxes / 4 + offsets));
+      cell_bytes = 2 * offsets;
+    }
+  }
+  L.cells = o; o = lm_align16(o + cell_bytes);
   L.cell_obs = o; o = lm_align16(o + 2 * (size_t)L.max_entries);
   if (threads == 0) {
     L.slots = o; o = lm_align16(o + 28 * (size_t)a.m.n_joints * nc);
@@ -1144,7 +1161,7 @@ __device__ void lm_stage(const LmArgs& a, unsigned char* smem_raw, const LmLayou
     __syncthreads();
   }
 
-  int* cell_int = L.recs ? scratch + ((a.w.Ms + 3) & ~3) : cell_start;
+  int* cell_int = L.cell_ints ? scratch + L.cell_ints : cell_start;
   if (sh.grid_on) {
     if (tid < 32) obstacle_grid_bounds(ws4, a.w.Ms, sh.rmax, a.grid_n, sh.glo, sh.ginv);
     __syncthreads();
@@ -1165,8 +1182,14 @@ __device__ void lm_stage(const LmArgs& a, unsigned char* smem_raw, const LmLayou
     }
     if (L.recs) {
       // the seed-group kernels keep the offsets (at most 16,384) in 16 bits
+      // (a round writes over ints that it or an earlier one has read, should they lie in the same place)
       unsigned short* cell16 = reinterpret_cast<unsigned short*>(cell_start);
-      for (int c = tid; c <= obstacle_grid_cells(sh.grid_n); c += nth) cell16[c] = (unsigned short)cell_int[c];
+      const int last = obstacle_grid_cells(sh.grid_n);
+      for (int c0 = 0; c0 <= last; c0 += nth) {
+        const int v = c0 + tid <= last ? cell_int[c0 + tid] : 0;
+        __syncthreads();
+        if (c0 + tid <= last) cell16[c0 + tid] = (unsigned short)v;
+      }
       __syncthreads();
     }
   }
@@ -1887,8 +1910,11 @@ __global__ void __launch_bounds__(128) verify_select_kernel(VerifyArgs a) {
 static size_t lm_smem_bytes(const LmArgs& a, int tps) { return lm_layout(a, tps).total; }
 
 // Blocks per SM that shared memory admits (at most the 4 of the small
-// register budget).
-static int lm_blocks_per_sm(size_t smem) { return (int)std::min<size_t>(4, (228 * 1024) / (smem + 1024)); }
+// register budget; none past the size that is refused).
+constexpr size_t kLmSmemMax = 220 * 1024;
+static int lm_blocks_per_sm(size_t smem) {
+  return smem > kLmSmemMax ? 0 : (int)std::min<size_t>(4, (228 * 1024) / (smem + 1024));
+}
 
 // The fine default grid (lm_grid_option) only where its larger cell lists
 // keep the blocks per SM that the default resolution admits; else the
@@ -1931,7 +1957,7 @@ static int launch_lm_t(const LmArgs& a0, cudaStream_t st) {
   lm_fit_grid(a, TPS);
   const int threads = a.spb * TPS;
   const size_t smem = lm_smem_bytes(a, TPS);
-  PK_CHECK_CAP(smem <= 220 * 1024, "LM working set (%zu B of shared memory) too large", smem);
+  PK_CHECK_CAP(smem <= kLmSmemMax, "LM working set (%zu B of shared memory) too large", smem);
   dim3 grid((a.Sd + a.spb - 1) / a.spb, a.P);
   // The 4-block register budget (spills) only where shared memory admits 3
   // or more blocks per SM and the grid needs more than 2 blocks per SM.
@@ -1971,7 +1997,7 @@ static int launch_lm_trial(LmArgs a, cudaStream_t st) {
   a.spb = 6 * (threads / 32);  // 6 groups of 5 lanes per warp
   lm_fit_grid(a, 1, threads);
   const size_t smem = lm_layout(a, 1, threads).total;
-  PK_CHECK_CAP(smem <= 220 * 1024, "LM working set (%zu B of shared memory) too large", smem);
+  PK_CHECK_CAP(smem <= kLmSmemMax, "LM working set (%zu B of shared memory) too large", smem);
   auto kern = lm_trial_kernel<MAXA, MAXEE>;
   if (int s = set_smem_limit((const void*)kern, smem)) return s;
   dim3 grid((a.Sd + a.spb - 1) / a.spb, a.P);
@@ -2302,7 +2328,7 @@ static int launch_seed_group_body(const BatchCall& b, int body, cudaStream_t st,
     }
   }
   if (!any || b.n_items == 0) return PK_OK;
-  PK_CHECK_CAP(smem <= 220 * 1024, "LM working set (%zu B of shared memory) too large", smem);
+  PK_CHECK_CAP(smem <= kLmSmemMax, "LM working set (%zu B of shared memory) too large", smem);
   B.n_classes = b.n_classes;
   B.items = b.items;
   B.n_items = b.n_items;

@@ -63,6 +63,21 @@ def test_lm_rejects_dof_beyond_capacity(lib):
     assert st == _lib.PK_ERR_INVALID                  # no end-effector
 
 
+@pytest.mark.parametrize("seeds_per_block,threads,grid,most", [(32, 1, 0, 8992), (32, 1, 14, 8544), (4, 8, 14, 8448),
+                                                               (128, 1, 16, 8256), (32, 1, -1, 10720)])
+def test_lm_accepts_worlds_up_to_shared_memory(lib, seeds_per_block, threads, grid, most):
+    """The largest sphere worlds that one block holds (7 joints, 8 robot spheres): one more is refused for its
+    size.  Nothing runs: the 70,000 problems are past what a launch takes."""
+    opt = _lib.LmOptions(4, 50, 10, 1e-2, 0.1, 10, 1e-8, 1e-8, 1, 1e4, 0.02, threads, seeds_per_block, 0, 0, grid)
+    d = C.c_void_p(16)
+    for Ms, status in ((most, _lib.PK_ERR_CUDA), (most + 1, _lib.PK_ERR_CAPACITY)):
+        assert lib.pk_ls_ik_ex(None, C.byref(opt), *([d] * 25), 70000, 8, 7, 7, 1, 8, Ms, 0, 0, 0, 0) == status
+        assert (status == _lib.PK_ERR_CUDA) or b"shared memory" in lib.pk_last_error()
+    # 52 joints: the finer default grid does not fit, the coarser one does
+    opt = _lib.LmOptions(4, 50, 10, 1e-2, 0.1, 10, 1e-8, 1e-8, 1, 1e4, 0.02, 0, 128, 0, 0, 0)
+    assert lib.pk_ls_ik_ex(None, C.byref(opt), *([d] * 25), 70000, 8, 16, 52, 1, 6, 156, 1, 5, 0, 0) == _lib.PK_ERR_CUDA
+
+
 def test_self_sphere_rejects_negative(lib):
     d = C.c_void_p(16)
     assert lib.pk_collision_self_sphere(None, d, d, d, d, d, 4, -1, 8, 3) == _lib.PK_ERR_INVALID

@@ -165,6 +165,21 @@ def test_lm_obstacle_grid_resolution_leaves_results_unchanged(tps):
             assert np.mean(np.abs(a - b) <= 1e-4 * np.abs(b) + 1e-5) >= 0.95, grid
 
 
+@pytest.mark.parametrize("n_obstacles", [40, 600])
+def test_lm_grid_offsets_in_small_blocks(n_obstacles):
+    """Blocks of 32 seeds have few pose slots, and the grid's 16-bit offsets are made in the place of the 32-bit
+    ones: the bits are the same with every grid and without one."""
+    w = W.ik(P=2, Sd=40, n_obstacles=n_obstacles)
+    s = solver_for(w, max_iter=4, threads_per_seed=1, seeds_per_block=32)
+    base = None
+    for grid in (-1, 0, 1, 9, 14, 16):
+        s.opt.obstacle_grid = grid
+        c, e = s.run_lm(tt(w.target_T), tt(w.seeds))
+        if base is None:
+            base = c, e
+        assert torch.equal(c, base[0]) and torch.equal(e, base[1]), grid
+
+
 def test_lm_fp64_solve_rejects_other_mappings():
     w = small_ik(P=1, Sd=8)
     with pytest.raises(Exception, match="fp64_solve"):
