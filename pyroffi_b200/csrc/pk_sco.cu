@@ -133,10 +133,10 @@ __device__ __forceinline__ float group_sum(float v, unsigned gm) {
 }
 
 // (x, y, z) to unit length by the approximate reciprocal root and one Newton
-// step (about an ulp); 0 stays 0.
+// step (about an ulp); 0 where the square is 0 or subnormal (below 1.1e-19).
 __device__ __forceinline__ float3 unit_from(float x, float y, float z) {
   const float d2 = x * x + y * y + z * z;
-  float i = rsqrt_approx(d2 + 1e-30f);
+  float i = d2 >= FLT_MIN ? rsqrt_approx(d2) : 0.f;
   i = i * fmaf(-0.5f * d2, i * i, 1.5f);
   return make_float3(x * i, y * i, z * i);
 }

@@ -62,6 +62,25 @@ def test_analytic_jacobian_matches_fp64_differences(self_all):
     np.testing.assert_allclose(J.cpu().numpy(), oJ, atol=2e-4, rtol=1e-3)
 
 
+@pytest.mark.parametrize("q", [0.0, 1e-18, 1e-17, 1e-15, 1e-12, 1e-3])
+def test_gradients_stay_unit_next_to_a_centre(q):
+    """A sphere q along x from the centre of a sphere, the axis of a capsule and the face of a box without
+    thickness: the distances' gradients are 1 however small q is, and at 0 they are 0, 0 and 1."""
+    from pyroffi_b200.robot import RobotModel, RobotSpheres
+    m = RobotModel(twists=np.array([[1.0, 0, 0, 0, 0, 0]]), parent_tf=np.array([[1.0, 0, 0, 0, 0, 0, 0]]),
+                   parent_idx=[-1], act_idx=[0], mimic_mul=[1.0], mimic_off=[0.0], mimic_act_idx=[-1],
+                   parent_joint_indices=[-1, 0], lower=[-1.0], upper=[1.0])
+    sph = RobotSpheres(np.zeros((2, 1, 3), np.float32), np.array([[-1.0], [0.1]], np.float32))
+    world = W.empty_world()
+    world.spheres = np.array([[0, 0, 0, 0.2]], np.float32)
+    world.capsules = np.array([[0, -0.5, 0, 0, 0.5, 0, 0.1]], np.float32)
+    world.boxes = np.array([[0, 0, 0, 1, 0, 0, 0, 1, 0, 0, 0, 1, 0, 0.5, 0.5]], np.float32)
+    opt = ScoOptimizer(m, sph, world, np.zeros((0, 2)), device=DEV)
+    _, J, _ = opt.linearize(torch.full((1, 1), q, device=DEV))
+    want = [1.0, 1.0, 1.0] if q > 0 else [0.0, 0.0, 1.0]
+    np.testing.assert_allclose(J[0, 1:4, 0].cpu().numpy(), want, atol=1e-6)
+
+
 def test_fd_jacobian_as_the_reference_kernel():
     # central differences with the reference kernel's float32 step 1e-4
     w = scene()
