@@ -51,8 +51,8 @@ __device__ __forceinline__ ObsView world_view(const RowArgs& a, float* smem) {
 
 // A block's robot spheres packed per link into pairs: the spheres that exist,
 // moved to the front, spheres 2q and 2q + 1 of a link as float4 (x0, x1, y0, y1)
-// and (z0, z1, -r0, -r1); the odd slot of an odd count at 1e18 with -r = 1, so
-// its packed distances never win a minimum.
+// and (z0, z1, -r0, -r1); the odd slot of an odd count with -r = 1e30, so its
+// packed distances never win a minimum, wherever the obstacles are.
 __host__ __device__ __forceinline__ int link_pair_count(int S) { return (S + 1) >> 1; }
 
 // Packs `nc` configurations into dst (link n of configuration c at c * cstride
@@ -76,7 +76,7 @@ __device__ __forceinline__ void pack_link_pairs(float4* dst, int* counts, int nc
       if (r >= 0.f) put(centre(c, s, n), r);
     }
     counts[g] = (cnt + 1) >> 1;
-    if (cnt & 1) put(make_float3(1e18f, 1e18f, 1e18f), -1.f);
+    if (cnt & 1) put(make_float3(0.f, 0.f, 0.f), -1e30f);
   }
 }
 

@@ -181,6 +181,27 @@ def test_packed_links_with_nan_and_infinity():
         np.testing.assert_array_equal(a.cpu().numpy(), b.cpu().numpy())
 
 
+def test_packed_links_and_far_obstacles():
+    """Obstacles at the places that padding is given elsewhere (1e18, the origin): the empty half of a link's
+    last pair wins no minimum."""
+    rng = np.random.default_rng(4)
+    c, r = sphere_robot_batch(rng, 3, 3, 4, pad_frac=0.0)
+    c += 5.0                                                       # clear of the origin
+    far = 1e18 * np.ones((1, 3), np.float32)
+    world = [np.concatenate([far, [[0.0]]], 1), np.concatenate([far, far, [[0.1]]], 1),
+             np.concatenate([far, np.eye(3).reshape(1, 9), [[1.0, 1.0, 1.0]]], 1), np.zeros((0, 6))]
+    centers = np.ascontiguousarray(c.reshape(3, 12, 3).transpose(2, 0, 1))
+    red = lambda w: collision_world_sphere_reduced(tt(centers), tt(r.reshape(3, -1)), *[tt(x) for x in w], n=4)  # noqa: E731
+    assert (red(world) == 1e9).all()
+    world[0] = np.array([[0.0, 0.0, 0.0, 0.5]])
+    world[1] = world[1][:0]
+    ref = oc.world_sphere_reduced(c.reshape(3, 12, 3).astype(np.float64), r.reshape(3, -1), *[x.astype(np.float64) for x in
+                                                                                              world[:2]],
+                                  np.zeros((0, 15)), world[3], 4)
+    assert_distances(red([world[0], world[1], np.zeros((0, 15)), world[3]]).cpu().numpy(), ref,
+                     quantity="signed distance (collision_world_sphere_reduced)", case="obstacle at the origin")
+
+
 def test_reduced_rows_past_32_bits():
     """1,024 links against 8.4 million obstacles: more (link, obstacle) pairs than 32 bits count."""
     N, Ms = 1024, (1 << 23) + 8
