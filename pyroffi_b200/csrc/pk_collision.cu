@@ -71,9 +71,13 @@ __device__ __forceinline__ void pack_link_pairs(float4* dst, int* counts, int nc
       e[0] = p.x; e[2] = p.y; e[4] = p.z; e[6] = -r;
       ++cnt;
     };
+    // (the centre is read before the radius is known, so that the loads of
+    // several spheres are in flight together)
+#pragma unroll 4
     for (int s = 0; s < S; ++s) {
       const float r = radius(c, s, n);
-      if (r >= 0.f) put(centre(c, s, n), r);
+      const float3 p = centre(c, s, n);
+      if (r >= 0.f) put(p, r);
     }
     counts[g] = (cnt + 1) >> 1;
     if (cnt & 1) put(make_float3(0.f, 0.f, 0.f), -1e30f);
@@ -136,7 +140,8 @@ __host__ __device__ inline size_t link_rows_smem(int cpb, int N, int S) {
 // (configuration, link) pairs of the block, so they stay full whatever the
 // counts and never mix kinds; a lane holds its obstacle (four, for spheres,
 // nq columns apart so that loads and stores are consecutive over the lanes)
-// in registers while it runs over the link's sphere pairs.
+// in registers while it runs over the link's sphere pairs.  gridDim.y blocks
+// share the pairs of their configurations.
 __global__ void __launch_bounds__(256, 3) link_rows_kernel(LinkRowArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int N = a.N, S = a.S, SP = link_pair_count(S);
@@ -162,7 +167,7 @@ __global__ void __launch_bounds__(256, 3) link_rows_kernel(LinkRowArgs a) {
     ob.Ms = a.w.Ms; ob.Mc = a.w.Mc; ob.Mb = a.w.Mb; ob.Mh = a.w.Mh;
   }
   __syncthreads();
-  const int M = a.w.total(), rows = nc * N, tid = threadIdx.x, T = blockDim.x;
+  const int M = a.w.total(), rows = nc * N, tid = blockIdx.y * blockDim.x + threadIdx.x, T = gridDim.y * blockDim.x;
   float* out = a.out + b0 * N * (long long)M;
 
   const int nq = (ob.Ms + 3) >> 2;
@@ -539,7 +544,10 @@ extern "C" int pk_collision_world_sphere_reduced(void* stream, const float* cent
   const size_t wsm = r.stage ? wbytes : 0;
   // a block counts its (row, obstacle) pairs of a kind (quads, for spheres) in
   // 32 bits, with room for the step past the last one
-  const long long most = (1LL << 31) - 1024, wide = std::max({(Ms + 3LL) / 4, (long long)Mc, (long long)Mb, (long long)Mh});
+  constexpr long long kMostSplits = 1024;
+  const long long most = (1LL << 31) - 256 * kMostSplits;
+  const long long quads = (Ms + 3LL) / 4, columns = quads + Mc + Mb + Mh;
+  const long long wide = std::max({quads, (long long)Mc, (long long)Mb, (long long)Mh});
   if (link_rows_smem(1, r.N, r.S) + wsm <= 200 * 1024 && (r.stage || aligned) && n * wide <= most) {
     // as many configurations per block (at most 8) as leave three blocks for
     // every SM and fit half of its shared memory
@@ -547,12 +555,33 @@ extern "C" int pk_collision_world_sphere_reduced(void* stream, const float* cent
     while (r.cpb > 1 && ((B + r.cpb - 1) / r.cpb < 3 * 148 || link_rows_smem(r.cpb, r.N, r.S) + wsm > 100 * 1024 ||
                          r.cpb * n * wide > most))
       r.cpb >>= 1;
-    const size_t smem = link_rows_smem(r.cpb, r.N, r.S) + wsm;
-    const long long blocks = (B + r.cpb - 1) / r.cpb;
-    PK_CHECK_CAP(blocks < (1LL << 31), "batch too large");
-    if (int st = set_smem_limit((const void*)link_rows_kernel, smem)) return st;
-    link_rows_kernel<<<(unsigned)blocks, 256, smem, (cudaStream_t)stream>>>(r);
-    return cuda_status(cudaGetLastError(), "link_rows_kernel launch");
+    // The row kernel stays the faster one, once the batch fills the GPU,
+    // - for few obstacles, which use a packed sphere once or in too few lanes:
+    //   20,000 configurations of 3 links x 100 spheres among 5 capsules 200 us
+    //   (packed 334), among 8 spheres 118 (348), 1 sphere 86 (149); 7 x 8, 1
+    //   sphere 22 (34); 100 x 3, 1 sphere 78 (99), but 8 spheres 170 (123);
+    // - for links of one sphere, half of each pair, in a world that it can
+    //   stage in a third of an SM and this one cannot at all: 2,048
+    //   configurations of 64 x 1 among 4,100 spheres 1,066 us (1,142).
+    const long long work = B * n * columns;
+    const bool few = columns == 1 ? work > 100000 || work * r.S > 4000000
+                                  : r.cpb * n * columns < 256 && work > 100000;
+    const bool half = r.S == 1 && !r.stage && wbytes <= 75 * 1024 && work > 100000000;
+    if (!few && !half) {
+      const size_t smem = link_rows_smem(r.cpb, r.N, r.S) + wsm;
+      const long long blocks = (B + r.cpb - 1) / r.cpb;
+      PK_CHECK_CAP(blocks < (1LL << 31), "batch too large");
+      // the columns of a few configurations are split over as many blocks as
+      // fill the GPU, those of a large world over four times as many, so that no
+      // last wave of long blocks leaves it idle (each packs its configurations):
+      // one configuration of 64 links x 1 sphere, 5,000 obstacles 109 us in one
+      // block, 37 in the row kernel; 2,048 with 4,100 obstacles 1,213 and 1,067
+      const long long pairs = r.cpb * n * wide, want = (pairs >= 32768 ? 4 : 1) * 3 * 148;
+      const long long splits = std::max(1LL, std::min({(want + blocks - 1) / blocks, pairs / 1024, kMostSplits}));
+      if (int st = set_smem_limit((const void*)link_rows_kernel, smem)) return st;
+      link_rows_kernel<<<dim3((unsigned)blocks, (unsigned)splits), 256, smem, (cudaStream_t)stream>>>(r);
+      return cuda_status(cudaGetLastError(), "link_rows_kernel launch");
+    }
   }
   return launch_rows<1>((cudaStream_t)stream, a);
 }

@@ -202,6 +202,31 @@ def test_packed_links_and_far_obstacles():
                      quantity="signed distance (collision_world_sphere_reduced)", case="obstacle at the origin")
 
 
+@pytest.mark.parametrize("B,N,S,Ms,Mc,Mb", [(20000, 3, 21, 1, 0, 0), (20000, 3, 21, 0, 5, 0), (20000, 7, 8, 8, 0, 0),
+                                            (2048, 64, 1, 3500, 0, 0), (1, 64, 1, 5003, 3, 2), (3, 30, 5, 4099, 0, 0),
+                                            (70, 9, 3, 0, 900, 0), (444, 40, 2, 3300, 1, 1)])
+def test_reduced_rows_by_size(B, N, S, Ms, Mc, Mb):
+    """Sizes on both sides of the rules that choose between the packed kernel, its rows split over several
+    blocks, and the row kernel: few obstacles in a large batch, links of one sphere, few configurations."""
+    rng = np.random.default_rng(B + N)
+    c, r = sphere_robot_batch(rng, B, S, N)
+    world = [W.random_sphere_world(rng, Ms) if Ms else np.zeros((0, 4)),
+             W.random_capsules(rng, Mc) if Mc else np.zeros((0, 7)),
+             W.random_boxes(rng, Mb, oriented=True) if Mb else np.zeros((0, 15)), np.zeros((0, 6))]
+    centers = np.ascontiguousarray(c.reshape(B, S * N, 3).transpose(2, 0, 1))
+    red = collision_world_sphere_reduced(tt(centers), tt(r.reshape(B, -1)), *[tt(x) for x in world], n=N)
+    rows = sorted({0, 1 % B, B // 2, B - 1})
+    ref = oc.world_sphere_reduced(c[rows].reshape(len(rows), S * N, 3).astype(np.float64), r[rows].reshape(len(rows), -1),
+                                  *[np.asarray(x, np.float32).astype(np.float64) for x in world], N)
+    assert_distances(red[rows].cpu().numpy(), ref, quantity="signed distance (collision_world_sphere_reduced)",
+                     case=f"{B} x {N} x {S}, {Ms} + {Mc} + {Mb}")
+    if B > 1000:  # the first ones again, in a batch that takes the packed kernel
+        k = 64
+        part = collision_world_sphere_reduced(tt(np.ascontiguousarray(centers[:, :k])), tt(r[:k].reshape(k, -1)),
+                                              *[tt(x) for x in world], n=N)
+        torch.testing.assert_close(red[:k], part, rtol=1e-6, atol=2e-6)
+
+
 def test_reduced_rows_past_32_bits():
     """1,024 links against 8.4 million obstacles: more (link, obstacle) pairs than 32 bits count."""
     N, Ms = 1024, (1 << 23) + 8
