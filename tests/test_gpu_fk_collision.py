@@ -227,6 +227,21 @@ def test_reduced_rows_by_size(B, N, S, Ms, Mc, Mb):
         torch.testing.assert_close(red[:k], part, rtol=1e-6, atol=2e-6)
 
 
+@pytest.mark.parametrize("B,N,S,P", [(5000, 64, 1, 1), (5000, 64, 1, 127), (5000, 64, 1, 128), (9000, 30, 3, 19),
+                                     (9000, 30, 3, 20), (7200, 7, 4, 1), (7200, 7, 8, 2)])
+def test_self_distances_by_size(B, N, S, P):
+    """Pair counts on both sides of the rule between the packed kernel and the one that is faster for few pairs
+    of links of few spheres, and robots of which 8 and 16 share a block."""
+    rng = np.random.default_rng(P)
+    c, r = sphere_robot_batch(rng, B, S, N)
+    pi, pj = rng.integers(0, N, P).astype(np.int32), rng.integers(0, N, P).astype(np.int32)
+    out = collision_self_sphere(tt(c), tt(r), tt(pi, torch.int32), tt(pj, torch.int32))
+    rows = [0, 7, 8, B // 2, B - 1]
+    ref = oc.self_sphere_full(c[rows].astype(np.float64), r[rows].astype(np.float64), pi, pj)
+    assert_distances(out[rows].cpu().numpy(), ref, quantity="signed distance (collision_self_sphere)",
+                     case=f"{B} x {N} x {S}, {P} pairs")
+
+
 def test_reduced_rows_past_32_bits():
     """1,024 links against 8.4 million obstacles: more (link, obstacle) pairs than 32 bits count."""
     N, Ms = 1024, (1 << 23) + 8
