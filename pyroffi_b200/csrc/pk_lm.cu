@@ -117,8 +117,11 @@ __host__ __device__ __forceinline__ int lm_ms_pad(int Ms, int tps) {
   return ((Ms + chunk - 1) / chunk) * chunk;
 }
 
-// Self-pair groups per chunk of the warp item list (one lane per seed).
-constexpr int kSelfChunk = 4;
+// Self-pair groups per chunk of the warp item list (one lane per configuration).
+// With trial lanes 4, which leaves room for two blocks per SM; else 16, whose
+// longer lists split evenly over the warp: 1,500 pairs in blocks of 32 seeds
+// 3,884 us per launch of 32 seeds, 4,298 with 4.
+__host__ __device__ __forceinline__ constexpr int self_chunk(int trial_lanes) { return trial_lanes > 1 ? 4 : 16; }
 
 // Seeds per block of the 16-wide one-lane kernel by default: the 16-DOF /
 // 2-EE register state takes the whole register file at 2 blocks of 128
@@ -182,9 +185,9 @@ __host__ __device__ inline LmLayout lm_layout(const LmArgs& a, int tps, int thre
   L.pair4 = o; o = lm_align16(o + (threads > 0 ? 16 * (size_t)n_self : 0));
   L.prec = o; o = lm_align16(o + (threads == 0 ? 64 * (size_t)n_self : 0));
   L.pgstart = o; o = lm_align16(o + (threads == 0 ? 4 * (size_t)(n_self + 2) : 0));
-  // one lane per seed: per warp, the self-pair item list (kSelfChunk * 32 u16)
-  // and the item sums (kSelfChunk * 32 floats)
-  L.wscr = o; o = lm_align16(o + ((threads == 0 && tps == 1 && n_self > 0) ? (size_t)(nc / 32) * kSelfChunk * 32 * 6 : 0));
+  // one lane per configuration: per warp, the self-pair item list (self_chunk *
+  // 32 u16) and the item sums (self_chunk * 32 floats)
+  L.wscr = o; o = lm_align16(o + ((threads == 0 && tps == 1 && n_self > 0) ? (size_t)(nc / 32) * self_chunk(a.trial_lanes) * 32 * 6 : 0));
   L.recs = threads == 0 ? 1 : 0;
   L.gjoint = o; o = lm_align16(o + 8 * (size_t)(n_self + 1));
   L.gstart = o; o = lm_align16(o + 4 * (size_t)(n_self + 2));
@@ -324,7 +327,8 @@ __device__ __forceinline__ void narrow_world(const PenaltyCtx& c, const Pose& T,
 // added to pen (the even and the odd pairs' terms add up apart): one relative transform T_x^-1 T_y (rotation
 // conj(q_x) q_y as a matrix M, translation u = R_x^T (t_y - t_x)), then per
 // pair |c_a - (M c_b + u)| from the joint-frame records, two pairs per
-// packed FP32x2 operation.
+// packed FP32x2 operation, UNROLL of those at a time.
+template <int UNROLL>
 __device__ __forceinline__ void group_pairs(const PenaltyCtx& c, const PoseSlots& ps, int gi, float& pen) {
   const int2 ja = c.gjoint[gi];
   const Pose A = ps.load(c.jlist[ja.x]);
@@ -350,6 +354,7 @@ __device__ __forceinline__ void group_pairs(const PenaltyCtx& c, const PoseSlots
   // two pairs per packed FP32x2 operation: e = M c_b + u - c_a
   float2 sum = make_float2(0.f, 0.f);
   const int q1 = c.pgstart[gi + 1];
+#pragma unroll UNROLL
   for (int q = c.pgstart[gi]; q < q1; q += 2) {
     const float4 r0 = c.prec[2 * q], r1 = c.prec[2 * q + 1], r2 = c.prec[2 * q + 2], r3 = c.prec[2 * q + 3];
     const float2 bx = make_float2(r2.x, r2.y), by = make_float2(r2.z, r2.w), bz = make_float2(r3.x, r3.y);
@@ -384,13 +389,13 @@ __device__ __forceinline__ void self_share(const PenaltyCtx& c, const PoseSlots&
     while (mask) {
       const int gi = g0 + __ffs(mask) - 1;
       mask &= mask - 1u;
-      group_pairs(c, ps, gi, pen);
+      group_pairs<1>(c, ps, gi, pen);
     }
   }
 }
 
 // Self pairs of the 32 configurations of a warp (TPS == 1), all 32 lanes
-// together.  Per chunk of kSelfChunk groups, each lane culls the groups for
+// together.  Per chunk of CHUNK groups, each lane culls the groups for
 // its own configuration (none when !need); the surviving (lane, group) items
 // go into the warp's list in (group, lane) order; lane l takes items l, l +
 // 32, ... and writes each item's sum (its pairs in pair order) to
@@ -398,27 +403,31 @@ __device__ __forceinline__ void self_share(const PenaltyCtx& c, const PoseSlots&
 // group order.  The result does not depend on which lane took which item, and
 // the work of a chunk is spread over the warp instead of following the lane
 // with the most surviving groups.  slots_w: the pose slots of the warp's first
-// configuration.  The culls' loads are issued four groups at a time.
+// configuration.
+template <int CHUNK, bool B4>
 __device__ __forceinline__ void self_warp(const PenaltyCtx& c, const PoseSlots& ps, float* slots_w, int spb, bool need,
                                           float& pen, unsigned short* list, float* res) {
+  constexpr int STEP = B4 || CHUNK == 4 ? 4 : 1;  // culls with their loads in flight together
   const int lane = threadIdx.x & 31;
-  for (int g0 = 0; g0 < c.n_groups; g0 += kSelfChunk) {
-    const int nc = min(kSelfChunk, c.n_groups - g0);
+  for (int g0 = 0; g0 < c.n_groups; g0 += CHUNK) {
+    const int nc = min(CHUNK, c.n_groups - g0);
     unsigned mine = 0u;
     int n_items = 0;
     if (need) {
-      float d2[kSelfChunk], rr[kSelfChunk];
+      for (int i0 = 0; i0 < nc; i0 += STEP) {
+        float d2[STEP], rr[STEP];
 #pragma unroll
-      for (int u = 0; u < kSelfChunk; ++u) {
-        const int2 ja = c.gjoint[g0 + min(u, nc - 1)];
-        const float3 Bx = slot_centre(c, ps, ja.x), By = slot_centre(c, ps, ja.y);
-        const float dx = Bx.x - By.x, dy = Bx.y - By.y, dz = Bx.z - By.z;
-        rr[u] = c.jb[ja.x].w + c.jb[ja.y].w + c.margin;
-        d2[u] = dx * dx + dy * dy + dz * dz;
+        for (int u = 0; u < STEP; ++u) {
+          const int2 ja = c.gjoint[g0 + min(i0 + u, nc - 1)];
+          const float3 Bx = slot_centre(c, ps, ja.x), By = slot_centre(c, ps, ja.y);
+          const float dx = Bx.x - By.x, dy = Bx.y - By.y, dz = Bx.z - By.z;
+          rr[u] = c.jb[ja.x].w + c.jb[ja.y].w + c.margin;
+          d2[u] = dx * dx + dy * dy + dz * dz;
+        }
+#pragma unroll
+        for (int u = 0; u < STEP; ++u)
+          if (i0 + u < nc && d2[u] < rr[u] * fabsf(rr[u])) mine |= 1u << (i0 + u);
       }
-#pragma unroll
-      for (int u = 0; u < kSelfChunk; ++u)
-        if (u < nc && d2[u] < rr[u] * fabsf(rr[u])) mine |= 1u << u;
     }
     for (int i = 0; i < nc; ++i) {
       const bool sv = (mine >> i) & 1u;
@@ -431,7 +440,7 @@ __device__ __forceinline__ void self_warp(const PenaltyCtx& c, const PoseSlots& 
       const int item = list[k];
       const int o = item >> 8, i = item & 255;
       float part = 0.f;
-      group_pairs(c, PoseSlots{slots_w + o, spb}, g0 + i, part);
+      group_pairs<CHUNK == 4 ? 1 : 2>(c, PoseSlots{slots_w + o, spb}, g0 + i, part);
       res[i * 32 + o] = part;
     }
     __syncwarp();
@@ -478,7 +487,7 @@ __device__ __forceinline__ void self_warp(const PenaltyCtx& c, const PoseSlots& 
 // survivors are the same, but the compiler may contract a distance or a
 // hinge sum differently in the two forms (one ulp in about 1 of 2,000
 // outputs was seen).
-template <int TPS, bool B4>
+template <int TPS, bool B4, int CHUNK>
 __device__ float penalty_share(const PenaltyCtx& c, const PoseSlots& ps, int t, unsigned gmask, bool need,
                                float* slots_w, int spb, unsigned short* wlist, float* wres) {
   float pen = 0.f;
@@ -612,7 +621,7 @@ __device__ float penalty_share(const PenaltyCtx& c, const PoseSlots& ps, int t, 
   }
   if (TPS == 1 && c.n_groups > 0) {
     __syncwarp();  // other lanes read this lane's slots
-    self_warp(c, ps, slots_w, spb, need, pen, wlist, wres);
+    self_warp<CHUNK, B4>(c, ps, slots_w, spb, need, pen, wlist, wres);
   }
   __syncwarp(gmask);
   return pen;
@@ -1254,15 +1263,15 @@ __device__ __forceinline__ void lm_seed_groups(const LmArgs& a, unsigned char* s
   }
   float* const slots_w = slots + (cf & ~31);  // one lane per configuration: the pose slots of the warp's first one
   unsigned short* const wlist =
-      reinterpret_cast<unsigned short*>(smem_raw + L.wscr) + (size_t)(tid >> 5) * kSelfChunk * 32 * 3;
-  float* const wres = reinterpret_cast<float*>(wlist + kSelfChunk * 32);
+      reinterpret_cast<unsigned short*>(smem_raw + L.wscr) + (size_t)(tid >> 5) * self_chunk(TL) * 32 * 3;
+  float* const wres = reinterpret_cast<float*>(wlist + self_chunk(TL) * 32);
 
   // TPS == 1: called by every lane (collective); TPS > 1: by the lanes of
   // seeds that need it
   auto penalty = [&](bool need) -> float {
     if (!use_coll) return 0.f;
     if (TPS > 1 && !need) return 0.f;
-    const float share = penalty_share<TPS, B4>(pc, ps, t, gmask, need, slots_w, ncf, wlist, wres);
+    const float share = penalty_share<TPS, B4, self_chunk(TL)>(pc, ps, t, gmask, need, slots_w, ncf, wlist, wres);
     return a.coll_w * group_sum<TPS>(share, gmask);
   };
   // Every lane of the group computes the FK (same values); lane 0 stores it.
