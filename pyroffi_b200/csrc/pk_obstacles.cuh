@@ -417,7 +417,7 @@ __device__ __forceinline__ void near_of_kind(const ObsView& ob, Index index, int
   for (int k0 = lane; k0 < count; k0 += 32 * stride) {
     unsigned mask = 0u;
     const int n = min(32, (count - k0 + stride - 1) / stride);
-#pragma unroll 4
+#pragma unroll (KIND == 0 ? 4 : 1)
     for (int i = 0; i < n; ++i)
       if (obstacle_near<KIND>(ob, index(k0 + i * stride), B, R, margin)) mask |= 1u << i;
     while (mask) {

@@ -71,6 +71,8 @@ __device__ __forceinline__ bool box_orthonormal(const float* b) {
 
 // Obstacles that a warp's candidate list has room for: all but the halfspaces.
 __host__ __device__ __forceinline__ int listed(const WorldArgs& w) { return w.Ms + w.Mc + w.Mb; }
+// A kind is listed from this many obstacles per lane of a waypoint on.
+constexpr int kListMin = 8;
 
 // Warps of a block; two lanes for each of up to 8 waypoints are half a warp.
 __host__ __device__ __forceinline__ int traj_warps(int nth) { return (nth + 31) >> 5; }
@@ -141,7 +143,7 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
   }
   bool balls = true;
   for (int k = tid; k < ob.Mb; k += nth) balls = balls && box_orthonormal(ob.box + 15 * k);
-  const bool list_boxes = __syncthreads_and(balls) && a.list;  // else every box is tested
+  const bool list_boxes = __syncthreads_and(balls);  // else every box is tested
 
   constexpr bool want_grad = GRAD;
   const float margin = a.margin;
@@ -226,14 +228,24 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
       // testing every obstacle was most of the kernel's work: cost and gradient
       // launches of 512 x 64 x 7 among 288 obstacles 293 -> 205 us with the
       // spheres listed, 205 -> 180 with the capsules and boxes listed too and the
-      // cost apart from the gradient (five CHOMP iterations 3069 -> 2554)
-      const float3 bl3 = make_float3(warp_min_of(wm, B.x), warp_min_of(wm, B.y), warp_min_of(wm, B.z));
-      const float3 bh3 = make_float3(warp_max_of(wm, B.x), warp_max_of(wm, B.y), warp_max_of(wm, B.z));
+      // cost apart from the gradient (five CHOMP iterations 3069 -> 2554).  Of a
+      // kind with fewer than 8 obstacles per lane of a waypoint the lanes test all
+      // (296 x 64 among 5 capsules 53 us, listed 56), and so do warps with lanes of
+      // fewer than four waypoints, which share the listing among too few (64 x 33,
+      // one waypoint in the last warp, among 128 spheres 46 us, listed 62).
       const int lane = tid & 31, step = __popc(wm);
       int n_cand = 0;
+      const bool list = a.list && step >= 4 * TG;
+      const bool list0 = list && ob.Ms >= kListMin * TG, list1 = list && ob.Mc >= kListMin * TG,
+                 list2 = list && list_boxes && ob.Mb >= kListMin * TG;
+      float3 bl3 = B, bh3 = B;
+      if (list) {
+        bl3 = make_float3(warp_min_of(wm, B.x), warp_min_of(wm, B.y), warp_min_of(wm, B.z));
+        bh3 = make_float3(warp_max_of(wm, B.x), warp_max_of(wm, B.y), warp_max_of(wm, B.z));
+      }
       // lists obstacles base, base + 1, ... (ball(k): the bounding sphere of the k-th); returns their number
-      auto list_kind = [&](bool list, int base, int count, auto ball) {
-        if (!list) return count;
+      auto list_kind = [&](bool on, int base, int count, auto ball) {
+        if (!on) return count;
         const int first = n_cand;
         for (int k0 = 0; k0 < count; k0 += step) {
           const int k = k0 + lane;
@@ -253,16 +265,15 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
         return n_cand - first;
       };
       const int b1 = ob.Ms, b2 = b1 + ob.Mc, b3 = b2 + ob.Mb;
-      const int n0 = list_kind(a.list, 0, ob.Ms, [&](int k) { return ob.sph[k]; });
-      const int n1 = list_kind(a.list, b1, ob.Mc, [&](int k) { return capsule_ball(ob.cap + 7 * k); });
-      const int n2 = list_kind(list_boxes, b2, ob.Mb, [&](int k) { return box_ball(ob.box + 15 * k); });
-      __syncwarp(wm);
-      near_of_kind<0>(ob, [&](int i) { return a.list ? (int)cand[i] : i; }, n0, B, bl.w, margin, gl, TG, narrow);
-      near_of_kind<1>(ob, [&](int i) { return a.list ? (int)cand[n0 + i] : b1 + i; }, n1, B, bl.w, margin, gl, TG, narrow);
-      near_of_kind<2>(ob, [&](int i) { return list_boxes ? (int)cand[n0 + n1 + i] : b2 + i; }, n2, B, bl.w, margin, gl,
-                      TG, narrow);
+      const int n0 = list_kind(list0, 0, ob.Ms, [&](int k) { return ob.sph[k]; }), c1 = n_cand;
+      const int n1 = list_kind(list1, b1, ob.Mc, [&](int k) { return capsule_ball(ob.cap + 7 * k); }), c2 = n_cand;
+      const int n2 = list_kind(list2, b2, ob.Mb, [&](int k) { return box_ball(ob.box + 15 * k); });
+      if (list) __syncwarp(wm);
+      near_of_kind<0>(ob, [&](int i) { return list0 ? (int)cand[i] : i; }, n0, B, bl.w, margin, gl, TG, narrow);
+      near_of_kind<1>(ob, [&](int i) { return list1 ? (int)cand[c1 + i] : b1 + i; }, n1, B, bl.w, margin, gl, TG, narrow);
+      near_of_kind<2>(ob, [&](int i) { return list2 ? (int)cand[c2 + i] : b2 + i; }, n2, B, bl.w, margin, gl, TG, narrow);
       near_of_kind<3>(ob, [=](int i) { return b3 + i; }, ob.Mh, B, bl.w, margin, gl, TG, narrow);
-      __syncwarp(wm);  // the next link's list goes in the same place
+      if (list) __syncwarp(wm);  // the next link's list goes in the same place
       if (want_grad) {
 #pragma unroll
         for (int o = 1; o < TG; o <<= 1) {
@@ -501,7 +512,7 @@ extern "C" int pk_traj_cost_grad(void* stream, const pk_traj_options* opt, const
   // the candidate lists where they cost no resident block
   a.list = 0;
   size_t smem = traj_smem(a, nth, TG);
-  if (listed(a.w) > 0) {
+  if (std::max(Ms, std::max(Mc, Mb)) >= kListMin * TG) {
     a.list = 1;
     const size_t with = traj_smem(a, nth, TG);
     auto per_sm = [&](size_t b) { return std::min<size_t>(512 / nth, (228 * 1024) / (b + 1024)); };  // 128 registers

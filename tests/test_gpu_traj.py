@@ -94,6 +94,29 @@ def test_boxes_with_short_axes(scale):
     np.testing.assert_allclose(tc.cost_and_grad(x)[0].cpu().numpy(), ref, rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("total", [700, 10000])
+def test_worlds_with_and_without_a_list(total):
+    """Spheres out of reach pad the world.  10,000 of them and two warps' lists of them are more than a block
+    holds, so that every obstacle is tested: cost and gradient as of the world without the padding."""
+    rng = np.random.default_rng(6)
+    w, _ = setup(Bt=3, T=9)
+    w.world.spheres = W.random_sphere_world(rng, 40, lo=-0.5, hi=0.5)
+    w.world.capsules = W.random_capsules(rng, 9)
+    w.world.boxes = W.random_boxes(rng, 9, oriented=True)
+    x = torch.as_tensor(w.traj, device=DEV)
+    make = lambda: TrajectoryCost(w.model, w.spheres, w.world, w.link_pairs, margin=w.margin, w_smooth=0.0,  # noqa: E731
+                                  w_acc=0.0, w_jerk=0.0, w_limits=0.0, w_coll=1.0, device=DEV)
+    c, g = make().cost_and_grad(x)
+    near = w.world.spheres
+    w.world.spheres = np.tile(np.array([[100.0, 0, 0, 0.1]], np.float32), (total, 1))
+    w.world.spheres[::total // len(near)][:len(near)] = near
+    padded = make()
+    c2, g2 = padded.cost_and_grad(x)
+    np.testing.assert_allclose(c2.cpu().numpy(), c.cpu().numpy(), rtol=1e-5, atol=1e-6)
+    np.testing.assert_allclose(padded.cost(x).cpu().numpy(), c.cpu().numpy(), rtol=1e-5, atol=1e-6)
+    np.testing.assert_allclose(g2.cpu().numpy(), g.cpu().numpy(), rtol=1e-4, atol=1e-4)
+
+
 def test_gradient_matches_finite_differences():
     w, tc = setup(Bt=3, T=12)
     x = torch.as_tensor(w.traj, device=DEV)
