@@ -26,7 +26,9 @@ int cuda_status(cudaError_t e, const char* where) {
 }
 
 int set_smem_limit(const void* kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return PK_OK;
+  // 48 KB need no attribute, but the kernels' static shared memory (16 to 352
+  // bytes where there is dynamic) counts among them
+  if (bytes <= 47 * 1024) return PK_OK;
   return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes),
                      "cudaFuncSetAttribute");
 }

@@ -117,6 +117,24 @@ def test_worlds_with_and_without_a_list(total):
     np.testing.assert_allclose(g2.cpu().numpy(), g.cpu().numpy(), rtol=1e-4, atol=1e-4)
 
 
+@pytest.mark.parametrize("n_boxes", [0, 1])
+def test_working_sets_around_48_kb(n_boxes, tmp_path, monkeypatch):
+    """Worlds that take a block's working set past 48 KB in steps of 32 bytes, through a copy of the library
+    whose kernels have not been launched with more before."""
+    import shutil
+
+    from pyroffi_b200 import _lib
+    w, _ = setup(Bt=2, T=33)
+    w.world.boxes = W.random_boxes(np.random.default_rng(0), n_boxes, oriented=True)
+    x = torch.as_tensor(w.traj, device=DEV)
+    monkeypatch.setattr(_lib, "LIB_PATH", type(_lib.LIB_PATH)(shutil.copy(_lib.LIB_PATH, tmp_path)))
+    monkeypatch.setattr(_lib, "_lib", None)
+    monkeypatch.setattr(_lib, "_fns", {})
+    for n in range(100, 420):
+        w.world.spheres = np.tile(np.array([[100.0, 0, 0, 0.1]], np.float32), (n, 1))
+        TrajectoryCost(w.model, w.spheres, w.world, w.link_pairs, device=DEV).cost(x)
+
+
 def test_gradient_matches_finite_differences():
     w, tc = setup(Bt=3, T=12)
     x = torch.as_tensor(w.traj, device=DEV)
