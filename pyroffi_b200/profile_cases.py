@@ -7,6 +7,8 @@ capture one warm launch.
     python -m pyroffi_b200.profile_cases lm 1 128    # the same with 1 lane per seed, 128 seeds per block
     python -m pyroffi_b200.profile_cases fkc1        # fused FK + collision, 65,536 configs, [B, K, M] output
     python -m pyroffi_b200.profile_cases fkc5        # fused FK + collision, 4,096 configs of the sweep robot, [B, N, M]
+    python -m pyroffi_b200.profile_cases fk          # batched FK, 100,003 configurations of the 29-DOF humanoid
+    python -m pyroffi_b200.profile_cases rows        # drop-in distances, 2,048 x 30 links x 12 spheres: world and self
     python -m pyroffi_b200.profile_cases wide        # warp-per-seed LM, 15-DOF bimanual, 64 problems x 64 seeds
     python -m pyroffi_b200.profile_cases traj        # trajectory cost + adjoint, 512 x 64 x 7
     python -m pyroffi_b200.profile_cases batch       # persistent mixed batch, 512 problems
@@ -22,9 +24,11 @@ from __future__ import annotations
 
 import sys
 
+import numpy as np
 import torch
 
 from . import workloads as W
+from .device import DeviceRobot
 
 
 def _lm(tps=0, spb=0):
@@ -42,12 +46,42 @@ def _lm(tps=0, spb=0):
 
 def _fkc(B, sweep):
     from .collision import fk_sphere_collision
-    from .device import DeviceRobot, DeviceSpheres, DeviceWorld
+    from .device import DeviceSpheres, DeviceWorld
     w = W.sweep(B=B) if sweep else W.fk_collision(B=B)
     dev = torch.device("cuda:0")
     R, S, Wd = DeviceRobot.upload(w.model, dev), DeviceSpheres.upload(w.spheres, dev), DeviceWorld.upload(w.world, dev)
     c = torch.as_tensor(w.cfg, device=dev)
     return lambda: fk_sphere_collision(R, S, Wd, c, per_sphere=not sweep, per_link=sweep, link_poses=not sweep)
+
+
+def _fk():
+    from .cuda_kernels import fk_cuda
+    from .robot import humanoid_tree
+    m = humanoid_tree(np.random.default_rng(5))
+    r = DeviceRobot.upload(m, "cuda:0")
+    g = torch.Generator(device="cuda:0").manual_seed(5)
+    cfg = 2.0 * torch.rand((100003, m.n_act), device="cuda:0", generator=g) - 1.0
+    return lambda: fk_cuda(cfg, *r.fk_args(), r.fk_level_starts, r.fk_level_joints)
+
+
+def _rows():
+    from .cuda_kernels import collision_self_sphere, collision_world_sphere_reduced
+    from .robot import humanoid_tree, random_spheres
+    rng = np.random.default_rng(5)
+    m = humanoid_tree(rng)
+    sph = random_spheres(m, rng, per_link_range=(4, 12), base_spheres=True)
+    B, N, S = 2048, m.n_links, sph.S
+    f = lambda a: torch.as_tensor(np.ascontiguousarray(a, np.float32), device="cuda:0")  # noqa: E731
+    g = torch.Generator(device="cuda:0").manual_seed(5)
+    links = 2.0 * torch.rand((B, 1, N, 3), device="cuda:0", generator=g) - 1.0
+    cen = (links + f(sph.centers).transpose(0, 1)[None]).contiguous()          # [B, S, N, 3]
+    rad = f(sph.radii).T[None].expand(B, -1, -1).contiguous()
+    soa, rk = cen.reshape(B, S * N, 3).permute(2, 0, 1).contiguous(), rad.reshape(B, S * N)
+    world = [f(W.random_sphere_world(rng, 201)), f(W.random_capsules(rng, 33)), f(W.random_boxes(rng, 32, oriented=True)),
+             f(np.array([[0, 0, 1, 0, 0, -1.2], [0, 0, 1, 0, 0, -1.3]]))]
+    pairs = torch.as_tensor(W.active_link_pairs(m, sph), dtype=torch.int32, device="cuda:0")
+    pi, pj = pairs[:, 0].contiguous(), pairs[:, 1].contiguous()
+    return lambda: (collision_world_sphere_reduced(soa, rk, *world, N), collision_self_sphere(cen, rad, pi, pj))
 
 
 def _wide():
@@ -132,7 +166,7 @@ def _chomp():
     return lambda: opt.run(x, x[0, 0], x[0, -1])
 
 
-CASES = {"lm": _lm, "fkc1": lambda: _fkc(65536, False), "fkc5": lambda: _fkc(4096, True), "wide": _wide,
+CASES = {"lm": _lm, "fkc1": lambda: _fkc(65536, False), "fkc5": lambda: _fkc(4096, True), "fk": _fk, "rows": _rows, "wide": _wide,
          "traj": _traj, "batch": _batch, "scolin": lambda: _sco("lin"), "scoinner": lambda: _sco("inner"),
          "sco": lambda: _sco("run"), "hjcd": _hjcd, "sqp": _sqp, "chomp": _chomp}
 
