@@ -143,10 +143,11 @@ typedef struct pk_lm_options {
   int32_t enable_collision;
   float collision_weight;
   float collision_margin;
-  int32_t threads_per_seed; /* 0 = default (1 lane, and up to 8 DOF / 1 EE a second one for the line-search
-                              trials where two such blocks fit an SM; 128 seeds per block up to 8 DOF / 1 EE,
-                              96 up to 16 DOF / 2 EEs); 1, 2, 4, 8 = lanes sharing one seed; 5 = one lane per line-search
-                              trial; 16, 32 = warp-per-seed body with that many lanes per seed */
+  int32_t threads_per_seed; /* 0 = default (1 lane, and up to 8 DOF / 1 EE, with seeds_per_block 0, fp64_solve 0 and
+                              no negative collision_weight, a second one for the line-search trials where two such
+                              blocks fit an SM; 128 seeds per block up to 8 DOF / 1 EE, 96 up to 16 DOF / 2 EEs);
+                              1, 2, 4, 8 = lanes sharing one seed; 5 = one lane per line-search trial; 16, 32 =
+                              warp-per-seed body with that many lanes per seed */
   int32_t seeds_per_block;  /* 0 = choose automatically */
   int32_t lanes_per_wide_seed; /* warp-per-seed body: lanes per seed, 16 (0 = default) or 32 */
   int32_t fp64_solve;       /* the damped step is solved through its 6 n_ee x 6 n_ee dual system

@@ -30,13 +30,15 @@ struct BatchCall {
 // but share a stream.  From the second on they are launched with programmatic
 // stream serialization: every block of a kernel lets the next one start as soon
 // as it runs (batch_trigger), so the next kernel's blocks move in where the
-// last items of the one before leave SMs idle, and a kernel ends only after the
-// one before it has (batch_join, at the end of every block), so what follows
-// on the stream waits for all of them.  Nothing waits on a kernel that is not
-// wholly resident or done: a dependent's blocks start only after every block
-// of the kernel before has.  512 problems of the mixed workload, 6 iterations:
-// 7038 -> 5691 us, the same bits (the three kernels ran one after another, each
-// with SMs idle for 12 to 39% of its time behind its last items).
+// last items of the one before leave SMs idle, and a kernel that follows
+// another ends only after it has (batch_join, at the end of every block), so
+// what follows on the stream waits for all of them.  lm_warp_kernel has no
+// batch_join: it is always the first (launch_seed_group_batch comes after it).
+// Nothing waits on a kernel that is not wholly resident or done: a dependent's
+// blocks start only after every block of the kernel before has.  512 problems
+// of the mixed workload, 6 iterations: 7038 -> 5691 us, the same bits (the
+// three kernels ran one after another, each with SMs idle for 12 to 39% of its
+// time behind its last items).
 __device__ __forceinline__ void batch_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void batch_join() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

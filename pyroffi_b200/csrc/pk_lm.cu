@@ -154,9 +154,10 @@ __host__ __device__ inline size_t lm_align16(size_t x) { return (x + 15) & ~size
 // spheres in pairs (float4 (x0, x1, y0, y1), (z0, z1, r0, r1); an odd joint
 // padded with a sphere of radius -1e9), and each self-pair group's pairs in
 // pairs (float4 (-ax0, -ax1, -ay0, -ay1), (-az0, -az1, rr0, rr1),
-// (bx0, bx1, by0, by1), (bz0, bz1, 0, 0) with rr = r_a + r_b + margin; an odd group padded with a pair that never hits).  The staging
-// scratch (self-pair key counts, obstacle boxes) overlays the per-seed area
-// before the seeds run.
+// (bx0, bx1, by0, by1), (bz0, bz1, 0, 0) with rr = r_a + r_b + margin; an odd
+// group padded with a pair that never hits).  The staging scratch (joint slots,
+// obstacle boxes, the grid's offsets as ints) overlays the per-seed area before
+// the seeds run.
 // threads > 0: trial-lane kernel (per-lane pose slots for `threads` lanes,
 // per-seed sphere positions).
 __host__ __device__ inline LmLayout lm_layout(const LmArgs& a, int tps, int threads = 0) {
@@ -299,9 +300,9 @@ __device__ __forceinline__ void hinge_sq(float d2, float rr, float& pen) {
 
 // Exact hinge terms of the sphere pairs [p0, p1) of a joint against world
 // sphere O (radius already + margin), with the obstacle centre moved into
-// the joint's frame (T: the joint's rotation and its bounding centre, jb) once: |R c_k + t - o| = |c_k - R^T (o - t)|; two
-// spheres per packed FP32x2 operation (the even and the odd spheres' terms add
-// up apart).
+// the joint's frame (T: the joint's rotation and its bounding centre, jb)
+// once: |R c_k + t - o| = |c_k - R^T (o - t)|; two spheres per packed FP32x2
+// operation (the even and the odd spheres' terms add up apart).
 __device__ __forceinline__ void narrow_world(const PenaltyCtx& c, const Pose& T, float4 jb, int p0, int p1, float4 O,
                                              float& pen) {
   float3 o = pose_apply_inv(T, make_float3(O.x, O.y, O.z));  // relative to the bounding centre
@@ -324,10 +325,10 @@ __device__ __forceinline__ void narrow_world(const PenaltyCtx& c, const Pose& T,
 }
 
 // Hinge terms of the pairs of self-pair group gi of one seed (poses in ps),
-// added to pen (the even and the odd pairs' terms add up apart): one relative transform T_x^-1 T_y (rotation
-// conj(q_x) q_y as a matrix M, translation u = R_x^T (t_y - t_x)), then per
-// pair |c_a - (M c_b + u)| from the joint-frame records, two pairs per
-// packed FP32x2 operation, UNROLL of those at a time.
+// added to pen (the even and the odd pairs' terms add up apart): one relative
+// transform T_x^-1 T_y (rotation conj(q_x) q_y as a matrix M, translation u =
+// R_x^T (t_y - t_x)), then per pair |c_a - (M c_b + u)| from the joint-frame
+// records, two pairs per packed FP32x2 operation, UNROLL of those at a time.
 template <int UNROLL>
 __device__ __forceinline__ void group_pairs(const PenaltyCtx& c, const PoseSlots& ps, int gi, float& pen) {
   const int2 ja = c.gjoint[gi];
@@ -491,7 +492,6 @@ template <int TPS, bool B4, int CHUNK>
 __device__ float penalty_share(const PenaltyCtx& c, const PoseSlots& ps, int t, unsigned gmask, bool need,
                                float* slots_w, int spb, unsigned short* wlist, float* wres) {
   float pen = 0.f;
-  const bool b4 = B4;
   if (need) {
     if (TPS > 1) __syncwarp(gmask);  // the seed's other lanes have read the positions (residual) that go
     for (int j = t; j < c.n_js; j += TPS) {
@@ -519,7 +519,7 @@ __device__ float penalty_share(const PenaltyCtx& c, const PoseSlots& ps, int t, 
         // candidate slot in which any lane has a survivor
         for (int e0 = c.cell_start[cell] + t; e0 < e1; e0 += 32 * TPS) {
           unsigned mask = 0u;
-          if (!b4) {
+          if (!B4) {
             for (int i = 0; i < 32 && e0 + i * TPS < e1; ++i) {
               const float4 O = c.ws[c.cell_obs[e0 + i * TPS]];
               const float rr = R + O.w;
@@ -2032,7 +2032,9 @@ static int launch_lm(LmArgs a, int tps, int spb, cudaStream_t st) {
   // threads_per_seed 5: the trial-lane kernel (5 lanes per seed, one
   // line-search trial each); 1, 2, 4, 8: the seed-group kernel with the
   // collision penalty split across that many lanes; 0: the fastest measured
-  // default, 1 lane x 128 seeds per block.  (16 and 32, the warp-per-seed
+  // default, one lane per configuration -- in the 8-wide kernel, unless
+  // seeds_per_block is given too, two trial lanes x 128 seeds per block where
+  // two such blocks fit an SM (launch_lm_t).  (16 and 32, the warp-per-seed
   // body, are routed by lm_common.)
   if (tps <= 0) {
     tps = 1;

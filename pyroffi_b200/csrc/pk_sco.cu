@@ -1126,16 +1126,14 @@ __global__ void __launch_bounds__(kWpMaxT) sco_inner_wp_kernel(ScoInnerArgs a) {
       }
     }
     wp_sum<5>(tc, red, buf);
-    int best = 0;
     float tb = tc[0], ab = alpha[0];
 #pragma unroll
     for (int i = 1; i < 5; ++i)
-      if (tc[i] < tb) { best = i; tb = tc[i]; ab = alpha[i]; }
+      if (tc[i] < tb) { tb = tc[i]; ab = alpha[i]; }
     const float suff = cost * (1.f - 1e-4f);
 #pragma unroll
     for (int i = 4; i >= 0; --i)
-      if (tc[i] < suff) { best = i; tb = tc[i]; ab = alpha[i]; }
-    (void)best;
+      if (tc[i] < suff) { tb = tc[i]; ab = alpha[i]; }
     const bool better = tb < best_cost;
 #pragma unroll
     for (int d = 0; d < NA; ++d) {
