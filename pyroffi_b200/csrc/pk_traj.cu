@@ -47,7 +47,7 @@ struct TrajArgs {
   long long B;
   int T, N, S, P;
   float margin, w_smooth, w_acc, w_jerk, w_limits, w_coll;
-  int list;               // keep each warp's world-sphere candidates in shared memory
+  int list;               // kinds of which each warp lists candidates in shared memory: 1 spheres, 2 capsules, 4 boxes
   const unsigned char* active;  // null, or trajectory b runs only when active[b % active_period]
   long long active_period;
 };
@@ -143,15 +143,17 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
   }
   bool balls = true;
   for (int k = tid; k < ob.Mb; k += nth) balls = balls && box_orthonormal(ob.box + 15 * k);
-  const bool list_boxes = __syncthreads_and(balls);  // else every box is tested
+  const bool list_boxes = __syncthreads_and(balls) && (a.list & 4);  // else every box is tested
 
   constexpr bool want_grad = GRAD;
   const float margin = a.margin;
   const unsigned lanes = nth < 32 ? (1u << nth) - 1u : 0xffffffffu;  // of every warp of the block
   for (int t0 = 0; t0 < T; t0 += ng) {
-    const int t = t0 + grp;
-    const unsigned wm = __ballot_sync(lanes, t < T);  // the warp's lanes at work: a prefix of it
-    if (t >= T) continue;  // the whole group skips
+    if (t0 + (tid & ~31) / TG >= T) continue;  // the whole warp skips
+    // past the last waypoint a group repeats that one, and writes nothing: its
+    // lanes help the warp to list
+    const bool live = t0 + grp < T;
+    const int t = live ? t0 + grp : T - 1;
     const PoseSlots ps{slots + grp, ng};
     if (gl == 0) fk_thread(jt, [&](int i) { return xs[t * n + i]; }, ps);
     float* L = lt + grp;
@@ -230,21 +232,16 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
       // spheres listed, 205 -> 180 with the capsules and boxes listed too and the
       // cost apart from the gradient (five CHOMP iterations 3069 -> 2554).  Of a
       // kind with fewer than 8 obstacles per lane of a waypoint the lanes test all
-      // (296 x 64 among 5 capsules 53 us, listed 56), and so do warps with lanes of
-      // fewer than four waypoints, which share the listing among too few (64 x 33,
-      // one waypoint in the last warp, among 128 spheres 46 us, listed 62).
-      const int lane = tid & 31, step = __popc(wm);
+      // (296 x 64 among 5 capsules 53 us, listed 56).
+      const int lane = tid & 31, step = min(nth, 32);
       int n_cand = 0;
-      const bool list = a.list && step >= 4 * TG;
-      const bool list0 = list && ob.Ms >= kListMin * TG, list1 = list && ob.Mc >= kListMin * TG,
-                 list2 = list && list_boxes && ob.Mb >= kListMin * TG;
       float3 bl3 = B, bh3 = B;
-      if (list) {
-        bl3 = make_float3(warp_min_of(wm, B.x), warp_min_of(wm, B.y), warp_min_of(wm, B.z));
-        bh3 = make_float3(warp_max_of(wm, B.x), warp_max_of(wm, B.y), warp_max_of(wm, B.z));
+      if (a.list) {
+        bl3 = make_float3(warp_min_of(lanes, B.x), warp_min_of(lanes, B.y), warp_min_of(lanes, B.z));
+        bh3 = make_float3(warp_max_of(lanes, B.x), warp_max_of(lanes, B.y), warp_max_of(lanes, B.z));
       }
       // lists obstacles base, base + 1, ... (ball(k): the bounding sphere of the k-th); returns their number
-      auto list_kind = [&](bool on, int base, int count, auto ball) {
+      auto list_kind = [&](int on, int base, int count, auto ball) {
         if (!on) return count;
         const int first = n_cand;
         for (int k0 = 0; k0 < count; k0 += step) {
@@ -258,22 +255,22 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
             // not "<": a NaN pose or obstacle stays a candidate, as without the list
             in = !(dx * dx + dy * dy + dz * dz >= rr * fabsf(rr));
           }
-          const unsigned m = __ballot_sync(wm, in);
+          const unsigned m = __ballot_sync(lanes, in);
           if (in) cand[n_cand + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(base + k);
           n_cand += __popc(m);
         }
         return n_cand - first;
       };
       const int b1 = ob.Ms, b2 = b1 + ob.Mc, b3 = b2 + ob.Mb;
-      const int n0 = list_kind(list0, 0, ob.Ms, [&](int k) { return ob.sph[k]; }), c1 = n_cand;
-      const int n1 = list_kind(list1, b1, ob.Mc, [&](int k) { return capsule_ball(ob.cap + 7 * k); }), c2 = n_cand;
-      const int n2 = list_kind(list2, b2, ob.Mb, [&](int k) { return box_ball(ob.box + 15 * k); });
-      if (list) __syncwarp(wm);
-      near_of_kind<0>(ob, [&](int i) { return list0 ? (int)cand[i] : i; }, n0, B, bl.w, margin, gl, TG, narrow);
-      near_of_kind<1>(ob, [&](int i) { return list1 ? (int)cand[c1 + i] : b1 + i; }, n1, B, bl.w, margin, gl, TG, narrow);
-      near_of_kind<2>(ob, [&](int i) { return list2 ? (int)cand[c2 + i] : b2 + i; }, n2, B, bl.w, margin, gl, TG, narrow);
+      const int n0 = list_kind(a.list & 1, 0, ob.Ms, [&](int k) { return ob.sph[k]; }), c1 = n_cand;
+      const int n1 = list_kind(a.list & 2, b1, ob.Mc, [&](int k) { return capsule_ball(ob.cap + 7 * k); }), c2 = n_cand;
+      const int n2 = list_kind(list_boxes, b2, ob.Mb, [&](int k) { return box_ball(ob.box + 15 * k); });
+      if (a.list) __syncwarp(lanes);
+      near_of_kind<0>(ob, [&](int i) { return (a.list & 1) ? (int)cand[i] : i; }, n0, B, bl.w, margin, gl, TG, narrow);
+      near_of_kind<1>(ob, [&](int i) { return (a.list & 2) ? (int)cand[c1 + i] : b1 + i; }, n1, B, bl.w, margin, gl, TG, narrow);
+      near_of_kind<2>(ob, [&](int i) { return list_boxes ? (int)cand[c2 + i] : b2 + i; }, n2, B, bl.w, margin, gl, TG, narrow);
       near_of_kind<3>(ob, [=](int i) { return b3 + i; }, ob.Mh, B, bl.w, margin, gl, TG, narrow);
-      if (list) __syncwarp(wm);  // the next link's list goes in the same place
+      if (a.list) __syncwarp(lanes);  // the next link's list goes in the same place
       if (want_grad) {
 #pragma unroll
         for (int o = 1; o < TG; o <<= 1) {
@@ -346,7 +343,7 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
     }
 #pragma unroll
     for (int o = 1; o < TG; o <<= 1) cw += __shfl_xor_sync(gm, cw, o);
-    if (gl == 0) {
+    if (gl == 0 && live) {
       wpc[t] = cw;
       if (a.wp_coll) a.wp_coll[b * T + t] = cw;
       if (want_grad) {
@@ -512,8 +509,9 @@ extern "C" int pk_traj_cost_grad(void* stream, const pk_traj_options* opt, const
   // the candidate lists where they cost no resident block
   a.list = 0;
   size_t smem = traj_smem(a, nth, TG);
-  if (std::max(Ms, std::max(Mc, Mb)) >= kListMin * TG) {
-    a.list = 1;
+  const int kinds = (Ms >= kListMin * TG ? 1 : 0) | (Mc >= kListMin * TG ? 2 : 0) | (Mb >= kListMin * TG ? 4 : 0);
+  if (kinds) {
+    a.list = kinds;
     const size_t with = traj_smem(a, nth, TG);
     auto per_sm = [&](size_t b) { return std::min<size_t>(512 / nth, (228 * 1024) / (b + 1024)); };  // 128 registers
     if (with <= 200 * 1024 && per_sm(with) >= per_sm(smem)) smem = with;
