@@ -51,8 +51,8 @@ LM_FMA_PIPE_PCT = 32.5
 # The same counts for the trajectory kernel's fused forward + backward launch on the 512 x 64 x 7 workload
 # (python -m pyroffi_b200.profile_cases traj) and for the fused FK + collision kernel on the sweep robot's
 # per-link rows (python -m pyroffi_b200.profile_cases fkc5, 4,096 configurations; per configuration).
-TRAJ_EXECUTED_FLOP_PER_LAUNCH = 614165205
-TRAJ_FMA_PIPE_PCT = 23.3
+TRAJ_EXECUTED_FLOP_PER_LAUNCH = 615166669
+TRAJ_FMA_PIPE_PCT = 24.8
 SWEEP_EXECUTED_FLOP_PER_CONFIG = 27802706944 / 4096
 SWEEP_FMA_PIPE_PCT = 60.4
 
