@@ -141,9 +141,10 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
     // R < 0 marks a link without spheres; the slack keeps the cull conservative
     lbnd[l] = cnt ? make_float4(cx, cy, cz, R + 1e-4f + 1e-5f * fabsf(R)) : make_float4(0.f, 0.f, 0.f, -1.f);
   }
-  bool balls = true;
-  for (int k = tid; k < ob.Mb; k += nth) balls = balls && box_orthonormal(ob.box + 15 * k);
-  const bool list_boxes = __syncthreads_and(balls) && (a.list & 4);  // else every box is tested
+  bool balls = (a.list & 4) != 0;
+  if (balls)
+    for (int k = nth - 1 - tid; k < ob.Mb; k += nth) balls = balls && box_orthonormal(ob.box + 15 * k);
+  const bool list_boxes = __syncthreads_and(balls);  // else every box is tested
 
   constexpr bool want_grad = GRAD;
   const float margin = a.margin;

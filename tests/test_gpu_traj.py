@@ -78,13 +78,16 @@ def test_listed_capsules_and_boxes(n):
 
 
 @pytest.mark.parametrize("scale", [(0.5, 0.5, 0.5), (1.0, 0.3, 1.0)])
-def test_boxes_with_short_axes(scale):
-    """Axes shorter than 1 stretch a box past its half lengths: none of it may be lost to the list's balls."""
+@pytest.mark.parametrize("n_boxes,every", [(12, 1), (40, 1), (40, 13)])
+def test_boxes_with_short_axes(scale, n_boxes, every):
+    """Axes shorter than 1, of all boxes or a few, stretch a box past its half lengths: none of it may be lost to
+    the balls of a list (32 boxes and more, here)."""
     rng = np.random.default_rng(8)
     w, _ = setup(Bt=2, T=9)
     w.world.spheres = w.world.spheres[:1]
-    w.world.boxes = W.random_boxes(rng, 12, oriented=True)
-    w.world.boxes[:, 3:12] = (w.world.boxes[:, 3:12].reshape(-1, 3, 3) * np.array(scale, np.float32)[:, None]).reshape(-1, 9)
+    w.world.boxes = W.random_boxes(rng, n_boxes, oriented=True)
+    short = w.world.boxes[every - 1::every]
+    short[:, 3:12] = (short[:, 3:12].reshape(-1, 3, 3) * np.array(scale, np.float32)[:, None]).reshape(-1, 9)
     tc = TrajectoryCost(w.model, w.spheres, w.world, w.link_pairs, margin=w.margin, w_smooth=0.0, w_acc=0.0,
                         w_jerk=0.0, w_limits=0.0, w_coll=1.0, device=DEV)
     x = torch.as_tensor(w.traj, device=DEV)
