@@ -611,13 +611,15 @@ extern "C" int pk_collision_self_sphere(void* stream, const float* centers, cons
   // pairs of links of up to three spheres, which do not repay the packing:
   // 100,000 configurations of 64 links x 1 sphere, 1 pair 46 us (packed 72), 100
   // pairs 108 (123), 500 pairs 331 (304); 100 x 3, 20 pairs 231 (314), 100 pairs
-  // 394 (384); 30 x 2, 5 pairs 45 (61), 50 pairs less packed; four spheres or
-  // more always less packed.
+  // 394 (384); 30 x 2, 5 pairs 45 (61).  With four spheres or more the packed
+  // kernel is the faster one from one pair on.
   const bool few = S <= 3 && (long long)P * S < 2LL * N && (size_t)S * N * sizeof(float4) <= 96 * 1024;
   if (!few && self_pairs_smem(1, N, S) <= 200 * 1024) {
     // as for the reduced rows; 16 configurations of a small robot
     int cpb = 16;
-    while (cpb > 1 && ((B + cpb - 1) / cpb < 3 * 148 || self_pairs_smem(cpb, N, S) > (cpb > 8 ? 20 : 56) * 1024)) cpb >>= 1;
+    while (cpb > 1 &&
+           ((B + cpb - 1) / cpb < 3 * 148 || self_pairs_smem(cpb, N, S) > (cpb > 8 ? 20 : 56) * 1024))
+      cpb >>= 1;
     const size_t smem = self_pairs_smem(cpb, N, S);
     const long long blocks = (B + cpb - 1) / cpb;
     PK_CHECK_CAP(blocks < (1LL << 31), "batch too large");

@@ -268,8 +268,10 @@ __global__ void __launch_bounds__(64 * TG, 8 / TG) traj_cost_kernel(TrajArgs a) 
       const int n2 = list_kind(list_boxes, b2, ob.Mb, [&](int k) { return box_ball(ob.box + 15 * k); });
       if (a.list) __syncwarp(lanes);
       near_of_kind<0>(ob, [&](int i) { return (a.list & 1) ? (int)cand[i] : i; }, n0, B, bl.w, margin, gl, TG, narrow);
-      near_of_kind<1>(ob, [&](int i) { return (a.list & 2) ? (int)cand[c1 + i] : b1 + i; }, n1, B, bl.w, margin, gl, TG, narrow);
-      near_of_kind<2>(ob, [&](int i) { return list_boxes ? (int)cand[c2 + i] : b2 + i; }, n2, B, bl.w, margin, gl, TG, narrow);
+      near_of_kind<1>(ob, [&](int i) { return (a.list & 2) ? (int)cand[c1 + i] : b1 + i; }, n1, B, bl.w, margin, gl, TG,
+                      narrow);
+      near_of_kind<2>(ob, [&](int i) { return list_boxes ? (int)cand[c2 + i] : b2 + i; }, n2, B, bl.w, margin, gl, TG,
+                      narrow);
       near_of_kind<3>(ob, [=](int i) { return b3 + i; }, ob.Mh, B, bl.w, margin, gl, TG, narrow);
       if (a.list) __syncwarp(lanes);  // the next link's list goes in the same place
       if (want_grad) {
